@@ -154,7 +154,7 @@ struct dfn_handle {
     // shared-geometry batch in FP64 (DFN_STORE_FP64_SHARED): one K, splits of
     // the columns, packed V of all members per stage
     bool s64 = false;
-    int s64_split = 1, s64_kps = 0, s64_nkc = 0, s64_rp = S64_MEM;
+    S64Plan s64_pl;
     double *s64_vt = nullptr;
     StepCtl *ctl = nullptr;
     StepCtl *h_ctl = nullptr;     // pinned mirror, B entries
@@ -396,24 +396,30 @@ static int launch_tc(dfn_handle *h, const double *Vbase, int vmul)
     return DFN_OK;
 }
 
-// Shared-geometry K.V in FP64: V of every member packed per column, then one
-// GEMM over (row tile, member tile, column split).
-static int launch_s64(dfn_handle *h, const double *Vbase, int vmul)
+typedef void (*s64_fn)(const double *, const double *, const Inst *, const StepCtl *, int, int64_t, int64_t, int,
+                       S64Plan, double *, double *);
+template <int MODE>
+static s64_fn pick_s64(int nt)
+{
+    static const s64_fn fns[S64_NT] = {s64_gemm_kernel<MODE, 1>, s64_gemm_kernel<MODE, 2>, s64_gemm_kernel<MODE, 3>,
+                                       s64_gemm_kernel<MODE, 4>, s64_gemm_kernel<MODE, 5>, s64_gemm_kernel<MODE, 6>,
+                                       s64_gemm_kernel<MODE, 7>, s64_gemm_kernel<MODE, 8>};
+    return fns[nt - 1];
+}
+
+// Shared-geometry K.V in FP64: V of every member into padded rows, then one
+// GEMM whose CTAs share the (row tile, member tile, column chunk) steps.
+static int launch_s64(dfn_handle *h, int mask, const double *Vbase, int vmul)
 {
     const Inst &I = h->hinst[0];
-    const int64_t nv = I.Np * h->s64_rp;
-    s64_pack_v_kernel<<<blocks_of(nv, 256), 256, 0, h->stream>>>(Vbase, vmul, h->inst, I.N, h->B, h->s64_rp, I.Np,
-                                                                 h->s64_vt);
+    const S64Plan &pl = h->s64_pl;
+    s64_pack_v_kernel<<<dim3(blocks_of(I.Np, 256), (unsigned)(8 * pl.nt * pl.mtiles)), 256, 0, h->stream>>>(
+        Vbase, vmul, h->inst, I.N, h->B, I.Np, h->s64_vt);
     h->launches++;
     CKL();
-    dim3 grid((unsigned)((I.N + S64_ROWS - 1) / S64_ROWS), (unsigned)(h->s64_rp / S64_MEM), (unsigned)h->s64_split);
-    const double *K = static_cast<const double *>(h->K);
-    if (h->mode == DFN_MODE_II)
-        s64_gemm_kernel<2><<<grid, S64_THREADS, s64_smem_bytes(2), h->stream>>>(
-            K, h->s64_vt, h->inst, I.N, I.Np, h->B, h->s64_rp, h->s64_kps, h->s64_nkc, h->partT, h->partN);
-    else
-        s64_gemm_kernel<3><<<grid, S64_THREADS, s64_smem_bytes(3), h->stream>>>(
-            K, h->s64_vt, h->inst, I.N, I.Np, h->B, h->s64_rp, h->s64_kps, h->s64_nkc, h->partT, h->partN);
+    const s64_fn fn = h->mode == DFN_MODE_II ? pick_s64<2>(pl.nt) : pick_s64<3>(pl.nt);
+    fn<<<(unsigned)pl.ctas, S64_THREADS, s64_smem_bytes(h->mode, pl.nt), h->stream>>>(
+        static_cast<const double *>(h->K), h->s64_vt, h->inst, h->ctl, mask, I.N, I.Np, h->B, pl, h->partT, h->partN);
     return DFN_OK;
 }
 
@@ -430,7 +436,7 @@ static int launch_gemv(dfn_handle *h, int mask, const double *Vbase, int vmul, b
     } else if (h->tc) {
         TRY(launch_tc(h, Vbase, vmul));
     } else if (h->s64) {
-        TRY(launch_s64(h, Vbase, vmul));
+        TRY(launch_s64(h, mask, Vbase, vmul));
     } else if (h->gemv_impl == 0) {
         gemv_tma_fn fn = pick_gemv_tma(h->mode, h->store);
         fn<<<(unsigned)ntiles, (TMA_CONSUMERS + 1) * 32, kTmaSmem, h->stream>>>(
@@ -1504,20 +1510,7 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
             return DFN_ERR_ARG;
         }
         const int64_t N0 = p0.nb_element;
-        if (h->s64) {
-            // column splits: the fewest that fill whole waves (three CTAs per SM)
-            h->s64_rp = ((count + S64_MEM - 1) / S64_MEM) * S64_MEM;
-            h->s64_nkc = (int)((N0 + S64_COLS - 1) / S64_COLS);
-            const int64_t tiles = ((N0 + S64_ROWS - 1) / S64_ROWS) * (h->s64_rp / S64_MEM);
-            const int64_t slots = (int64_t)h->sms * 3;
-            double best = -1.0;
-            for (int sp = 1; sp <= 16 && sp <= h->s64_nkc; sp++) {
-                const int64_t units = tiles * sp;
-                const double eff = (double)units / (double)(((units + slots - 1) / slots) * slots);
-                if (eff > best + 0.02) { best = eff; h->s64_split = sp; }
-            }
-            h->s64_kps = (h->s64_nkc + h->s64_split - 1) / h->s64_split;
-        }
+        if (h->s64) h->s64_pl = s64_plan(N0, count, h->sms);
     }
     if (h->tc) {
         const dfn_problem &p0 = probs[0];
@@ -1549,7 +1542,7 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
         I.Np = (h->hmat || h->tc) ? I.N : (h->s64 ? ((I.N + S64_COLS - 1) / S64_COLS) * S64_COLS
                                                  : ((I.N + CW - 1) / CW) * CW);
         I.eoff = eoff;
-        I.nchunk = h->hmat ? 1 : (h->tc ? h->tc_split : (h->s64 ? h->s64_split : I.Np / CW));
+        I.nchunk = h->hmat ? 1 : (h->tc ? h->tc_split : (h->s64 ? h->s64_pl.slots : I.Np / CW));
         I.kvec = h->s64 ? 0 : kvec;   // a shared-geometry batch has one matrix
         I.poff = poff;
         I.soff = soff;
@@ -1810,11 +1803,10 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
             assemble_kernel<3, 0><<<grid, 256, 0, h->stream>>>(I.N, I.Np, h->node, h->elem, h->tan, h->nrm, h->K);
         h->launches++;
         CKC(cudaGetLastError());
-        DALLOC(h->s64_vt, I.Np * h->s64_rp);
-        CKC(cudaFuncSetAttribute(s64_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)s64_smem_bytes(2)));
-        CKC(cudaFuncSetAttribute(s64_gemm_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)s64_smem_bytes(3)));
+        const S64Plan &pl = h->s64_pl;
+        DALLOC(h->s64_vt, I.Np * 8 * pl.nt * pl.mtiles);
+        CKC(cudaFuncSetAttribute(h->mode == 2 ? pick_s64<2>(pl.nt) : pick_s64<3>(pl.nt),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s64_smem_bytes(h->mode, pl.nt)));
     }
     std::vector<int4> tiles;
     for (int i = 0; i < count && !h->hmat && !h->tc && !h->s64; i++) {

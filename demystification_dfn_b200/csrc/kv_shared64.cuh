@@ -1,163 +1,277 @@
 // kv_shared64.cuh — FP64 K.V of a batch whose networks share one kernel
 // matrix (DFN_STORE_FP64_SHARED). The R slip-rate vectors of a stage meet the
 // same K, so K.V is a GEMM, C[k][m] = sum_l K[k][l] V_m[l] (rows k with their
-// shear and normal entries, members m), computed in FP64 on the CUDA cores
-// with K streamed from HBM once for all members. It is the FP64 counterpart
-// of the tensor-core batch (tc_gemm.cuh): same K sharing, FP64 products and
-// sums, so that the two isolate what the BF16 hi+lo tensor-core arithmetic
-// itself gains. (The reference has one network per process and no batch.)
+// shear and normal entries, members m), in FP64 with K streamed from HBM once
+// per member tile. It is the FP64 counterpart of the tensor-core batch
+// (tc_gemm.cuh): same K sharing, FP64 products and sums, so that the two
+// isolate what the BF16 hi+lo arithmetic itself gains. (The reference has one
+// network per process and no batch.)
+//
+// The products run on the FP64 matrix instructions (mma.sync m16n8k16.f64:
+// IEEE FP64 products and sums): the contraction is bound by the FP64 unit for
+// R >= 16 (16 flop per byte of K at R = 64), and against scalar FMAs one
+// instruction replaces 64 per lane and a fragment load serves 16 rows x 8
+// members.
 //
 // K is stored row-major, N rows of Np columns (Np = N padded to S64_COLS with
 // zero columns), {K_T, K_N} per column in mode II; the V of all members is
-// packed per stage into vt[l][m] (RP members padded to S64_MEM with zeros).
-// CTA tile: S64_ROWS rows x S64_MEM members; the columns of the CTA's split
-// pass through a two-buffer shared-memory pipeline (cp.async, 16 bytes per
-// copy) in chunks of S64_COLS. Thread (ty, tx) owns rows 2ty, 2ty+1 and
-// members 2tx, 2tx+1, 32+2tx, 33+2tx of the tile (so that a half-warp reads
-// 256 contiguous bytes of V): 8 shear (and 8 normal) accumulators. K rows
-// in shared memory are padded by 16 bytes, so the two rows a warp reads at
-// once fall in different banks.
-// Each split writes its partial sums to part[poff_m + split*N + k] (the
-// layout the stage kernel sums in fixed order), so results are
-// deterministic.
+// packed per stage into vt[m][l] (members padded to 8, columns to Np, zeros).
+// A CTA of four warps takes S64_ROWS rows (16 per warp) x 8 NT members (a
+// member tile; NT the smallest that covers R in the fewest tiles, so that
+// padding costs at most 7 members per tile) and streams the columns in chunks
+// of S64_COLS through a ring of shared-memory stages (cp.async, 16 bytes per
+// copy). Lane (g, t) of a warp holds rows g, g + 8 and columns t, t + 4,
+// t + 8, t + 12 of the chunk, which is the fragment order of the instruction;
+// the stage rows are padded so that a quarter-warp's 16-byte reads of K and a
+// half-warp's 8-byte reads of V cover all banks once.
+//
+// Split of the work: the (row tile, member tile, column chunk) steps form one
+// sequence that the CTAs of a single wave share evenly (CTA b takes steps
+// b*I/G .. (b+1)*I/G), so no last wave is partly empty and a row tile is cut
+// into few pieces. The piece of CTA b of a tile that starts in CTA b0 goes to
+// part[poff_m + (b - b0)*N + k]; the tile's last CTA zeroes the unused slots.
+// The stage kernel adds the slots in fixed order: deterministic.
+//
+// Measured at N = 8 272, R = 50, mode II: 0.879 -> 0.479 ms per K.V (scalar
+// FMAs on 32 x 64 tiles with 12 splits before; 32 TFLOP/s on the 56 padded
+// members, the instruction alone reaches 37). What mattered besides the
+// instruction: the loader's addresses advance by additions (recomputing them
+// with divisions per chunk left the matrix unit idle a third of the time,
+// 0.635 ms); more warps per scheduler (8 warps of half the members, or one
+// component each) gave nothing (0.630-0.666 ms).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-constexpr int S64_ROWS = 32;
-constexpr int S64_MEM = 64;
-constexpr int S64_COLS = 32;
-constexpr int S64_THREADS = 256;
+constexpr int S64_ROWS = 64;
+constexpr int S64_COLS = 16;
+constexpr int S64_THREADS = 128;
+constexpr int S64_NT = 8;                        // at most 8 tiles of 8 members per CTA
+constexpr int S64_MIN_STEPS = 8;                 // chunks a CTA gets at least
+constexpr int S64_VROW = S64_COLS + 4;           // doubles of a staged V row (160 bytes)
 
-// dynamic shared memory of one CTA: two buffers of K (rows x cols x {T,N})
-// and V (cols x members)
-__host__ __device__ constexpr size_t s64_smem_bytes(int mode)
+// doubles of a staged K row: 320 bytes (mode II) or 160
+__host__ __device__ constexpr int s64_krow(int mode) { return mode == 2 ? 2 * S64_COLS + 8 : S64_COLS + 4; }
+__host__ __device__ constexpr int s64_stage_doubles(int mode, int nt)
 {
-    return 2 * sizeof(double) * ((size_t)S64_ROWS * (S64_COLS * (mode == 2 ? 2 : 1) + 2) + (size_t)S64_COLS * S64_MEM);
+    return S64_ROWS * s64_krow(mode) + 8 * nt * S64_VROW;
+}
+// stages that fit two CTAs per SM, at most 6
+__host__ __device__ constexpr int s64_stages(int mode, int nt)
+{
+    return 108 * 1024 / (8 * s64_stage_doubles(mode, nt)) < 6 ? 108 * 1024 / (8 * s64_stage_doubles(mode, nt)) : 6;
+}
+__host__ __device__ constexpr size_t s64_smem_bytes(int mode, int nt)
+{
+    return sizeof(double) * (size_t)s64_stages(mode, nt) * s64_stage_doubles(mode, nt);
 }
 
-__device__ __forceinline__ void s64_cp16(void *smem_dst, const void *gmem_src)
+// The work of one launch: steps per row tile, steps in all, CTAs, tiles.
+struct S64Plan {
+    int nt = 1;            // tiles of 8 members per CTA
+    int mtiles = 1;        // member tiles
+    int nkc = 0;           // column chunks
+    int rtiles = 0;        // row tiles
+    int64_t steps = 0;     // rtiles * mtiles * nkc
+    int64_t ctas = 0;
+    int slots = 1;         // partial sums per element
+};
+// first step of CTA b, and the CTA that holds a step
+__host__ __device__ inline int64_t s64_first(int64_t b, int64_t steps, int64_t ctas) { return b * steps / ctas; }
+__host__ __device__ inline int64_t s64_cta_of(int64_t step, int64_t steps, int64_t ctas)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(
+    int64_t b = step * ctas / steps;
+    while (b + 1 < ctas && s64_first(b + 1, steps, ctas) <= step) b++;
+    while (s64_first(b, steps, ctas) > step) b--;
+    return b;
+}
+
+inline S64Plan s64_plan(int64_t N, int R, int sms)
+{
+    S64Plan p;
+    const int n8 = (R + 7) / 8;
+    p.mtiles = (n8 + S64_NT - 1) / S64_NT;
+    p.nt = (n8 + p.mtiles - 1) / p.mtiles;
+    p.nkc = (int)((N + S64_COLS - 1) / S64_COLS);
+    p.rtiles = (int)((N + S64_ROWS - 1) / S64_ROWS);
+    p.steps = (int64_t)p.rtiles * p.mtiles * p.nkc;
+    p.ctas = p.steps / S64_MIN_STEPS < 1 ? 1 : p.steps / S64_MIN_STEPS;
+    if (p.ctas > 2 * (int64_t)sms) p.ctas = 2 * (int64_t)sms;
+    for (int64_t t = 0; t < (int64_t)p.rtiles * p.mtiles; t++) {
+        const int64_t n = s64_cta_of((t + 1) * p.nkc - 1, p.steps, p.ctas) - s64_cta_of(t * p.nkc, p.steps, p.ctas) + 1;
+        if (n > p.slots) p.slots = (int)n;
+    }
+    return p;
+}
+
+// 16-byte copy; bytes = 0 writes zeros (src is not read then)
+__device__ __forceinline__ void s64_cp16(void *smem_dst, const void *gmem_src, uint32_t bytes)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(
                      __cvta_generic_to_shared(smem_dst))),
-                 "l"(gmem_src)
+                 "l"(gmem_src), "r"(bytes)
                  : "memory");
 }
 __device__ __forceinline__ void s64_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void s64_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// vt[l * RP + m] = V of member m at column l (zero beyond N and R); V of
-// member m is Vbase[vmul * eoff_m + l].
-__global__ void s64_pack_v_kernel(const double *__restrict__ Vbase, int vmul, const Inst *__restrict__ inst,
-                                  int64_t N, int R, int RP, int64_t Np, double *__restrict__ vt)
+// C (16 x 8) += A (16 x 4) B (4 x 8): a[0], a[1] rows g, g + 8 of column t,
+// b row t of column g, c rows g, g, g + 8, g + 8 of columns 2t, 2t + 1
+__device__ __forceinline__ void s64_mma(double c[4], const double a[2], double b)
 {
-    const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (idx >= Np * RP) return;
-    const int64_t l = idx / RP;
-    const int m = (int)(idx % RP);
-    vt[idx] = (l < N && m < R) ? Vbase[(int64_t)vmul * inst[m].eoff + l] : 0.0;
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a[0]), "d"(a[1]), "d"(b));
+}
+// Whether any of the R networks takes part in a launch (CTA-uniform; a
+// barrier): a shared K.V serves all of them or none.
+__device__ __forceinline__ bool any_takes_part(const StepCtl *ctl, int R, int mask)
+{
+    int on = 0;
+    for (int r = threadIdx.x; r < R; r += blockDim.x) on |= takes_part(ctl, r, mask);
+    return __syncthreads_or(on) != 0;
 }
 
-// grid (row tiles, member tiles, splits); split s covers column chunks
-// [s * kc_per_split, min(nkc, (s + 1) * kc_per_split)).
-template <int MODE>
-__global__ void __launch_bounds__(S64_THREADS) s64_gemm_kernel(const double *__restrict__ K,
-                                                               const double *__restrict__ vt,
-                                                               const Inst *__restrict__ inst, int64_t N, int64_t Np,
-                                                               int R, int RP, int kc_per_split, int nkc,
-                                                               double *__restrict__ partT,
-                                                               double *__restrict__ partN)
+// vt[m * Np + l] = V of member m at column l (zero beyond N and R); V of
+// member m is Vbase[vmul * eoff_m + l]. grid (ceil(Np / 256), RP)
+__global__ void s64_pack_v_kernel(const double *__restrict__ Vbase, int vmul, const Inst *__restrict__ inst,
+                                  int64_t N, int R, int64_t Np, double *__restrict__ vt)
 {
-    constexpr int CPE = (MODE == 2) ? 2 : 1;            // doubles per stored entry
-    constexpr int KROW = S64_COLS * CPE;                 // doubles per K row of a chunk
-    constexpr int KLD = KROW + 2;                        // padded row in shared memory
-    constexpr int KSZ = S64_ROWS * KLD, VSZ = S64_COLS * S64_MEM;
+    const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int m = blockIdx.y;
+    if (l >= Np) return;
+    vt[(int64_t)m * Np + l] = (l < N && m < R) ? Vbase[(int64_t)vmul * inst[m].eoff + l] : 0.0;
+}
+
+template <int MODE, int NT>
+__global__ void __launch_bounds__(S64_THREADS, 2)
+    s64_gemm_kernel(const double *__restrict__ K, const double *__restrict__ vt, const Inst *__restrict__ inst,
+                    const StepCtl *__restrict__ ctl, int mask, int64_t N, int64_t Np, int R, S64Plan pl,
+                    double *__restrict__ partT, double *__restrict__ partN)
+{
+    constexpr int CPE = (MODE == 2) ? 2 : 1;             // doubles per stored entry
+    constexpr int KLD = s64_krow(MODE);
+    constexpr int KSZ = S64_ROWS * KLD;
+    constexpr int STAGE = s64_stage_doubles(MODE, NT);
+    constexpr int ST = s64_stages(MODE, NT);
     extern __shared__ __align__(16) double s64_smem[];
-    double *Ks = s64_smem;                // [2][S64_ROWS][KLD]
-    double *Vs = s64_smem + 2 * KSZ;      // [2][S64_COLS][S64_MEM]
 
-    const int tid = threadIdx.x;
-    const int64_t r0 = (int64_t)blockIdx.x * S64_ROWS;
-    const int m0 = blockIdx.y * S64_MEM;
-    const int split = blockIdx.z;
-    const int kc0 = split * kc_per_split;
-    const int kc1 = (kc0 + kc_per_split < nkc) ? kc0 + kc_per_split : nkc;
-    const int ty = tid >> 4, tx = tid & 15;
+    if (!any_takes_part(ctl, R, mask)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int64_t s0 = s64_first(blockIdx.x, pl.steps, pl.ctas), s1 = s64_first(blockIdx.x + 1, pl.steps, pl.ctas);
 
-    double aT[2][4], aN[2][4];
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) { aT[i][j] = 0.0; aN[i][j] = 0.0; }
-
-    // one chunk of K rows and V columns into buffer b (16-byte copies; rows
-    // beyond N are zeros written directly)
-    auto load = [&](int b, int kc) {
-        const int64_t c0 = (int64_t)kc * S64_COLS;
-        double *kd = Ks + b * KSZ;
-        for (int p = tid; p < S64_ROWS * KROW / 2; p += S64_THREADS) {
-            const int row = p / (KROW / 2), q = p % (KROW / 2);
-            const int64_t gr = r0 + row;
-            double *dst = kd + row * KLD + 2 * q;
-            if (gr < N) s64_cp16(dst, K + (gr * Np + c0) * CPE + 2 * q);
-            else { dst[0] = 0.0; dst[1] = 0.0; }
-        }
-        double *vd = Vs + b * VSZ;
-        for (int p = tid; p < VSZ / 2; p += S64_THREADS) {
-            const int col = p / (S64_MEM / 2), q = p % (S64_MEM / 2);
-            s64_cp16(vd + col * S64_MEM + 2 * q, vt + (c0 + col) * RP + m0 + 2 * q);
-        }
-        s64_commit();
+    // Loader: the chunks of this CTA in order, each thread the same 16-byte
+    // copies of every chunk (K rows krow + i * KRS, V members mrow + i * MRS),
+    // from pointers that advance by one chunk and are set anew at a tile.
+    constexpr int KV = S64_COLS * CPE / 2, KRS = S64_THREADS / KV, KN = S64_ROWS / KRS;
+    constexpr int VV = S64_COLS / 2, MRS = S64_THREADS / VV, VN = (8 * NT + MRS - 1) / MRS;
+    const int krow = tid / KV, kq = tid % KV, mrow = tid / VV, mq = tid % VV;
+    const int64_t kstep = (int64_t)KRS * Np * CPE, vstep = (int64_t)MRS * Np;
+    const double *kp = nullptr, *vp = nullptr;
+    int lc = 0, ltile = 0, rows_left = 0;
+    auto set_tile = [&](int tile, int c) {
+        const int64_t r0 = (int64_t)(tile / pl.mtiles) * S64_ROWS, m0 = (int64_t)(tile % pl.mtiles) * (8 * NT);
+        ltile = tile;
+        lc = c;
+        rows_left = (int)(N - r0 < S64_ROWS ? N - r0 : S64_ROWS);
+        kp = K + ((r0 + krow) * Np + (int64_t)c * S64_COLS) * CPE + 2 * kq;
+        vp = vt + (m0 + mrow) * Np + (int64_t)c * S64_COLS + 2 * mq;
     };
-
-    if (kc0 < kc1) load(0, kc0);
-    for (int kc = kc0; kc < kc1; kc++) {
-        const int b = (kc - kc0) & 1;
-        if (kc + 1 < kc1) {
-            load(b ^ 1, kc + 1);
-            s64_wait<1>();
+    auto load = [&](int st) {
+        double *kd = s64_smem + st * STAGE + krow * KLD + 2 * kq;
+        double *vd = s64_smem + st * STAGE + KSZ + mrow * S64_VROW + 2 * mq;
+#pragma unroll
+        for (int i = 0; i < KN; i++) {
+            const bool on = krow + i * KRS < rows_left;   // rows beyond N: zeros
+            s64_cp16(kd + i * KRS * KLD, on ? kp + i * kstep : K, on ? 16u : 0u);
+        }
+#pragma unroll
+        for (int i = 0; i < VN; i++)
+            if (VN * MRS == 8 * NT || mrow + i * MRS < 8 * NT) s64_cp16(vd + i * MRS * S64_VROW, vp + i * vstep, 16u);
+        if (++lc == pl.nkc) {
+            set_tile(ltile + 1, 0);
         } else {
-            s64_wait<0>();
+            kp += S64_COLS * CPE;
+            vp += S64_COLS;
         }
-        __syncthreads();
-        const double *kb = Ks + b * KSZ + (2 * ty) * KLD;
-        const double *vb = Vs + b * VSZ + 2 * tx;
-#pragma unroll 8
-        for (int c = 0; c < S64_COLS; c++) {
-            const double2 v01 = *reinterpret_cast<const double2 *>(vb + c * S64_MEM);
-            const double2 v23 = *reinterpret_cast<const double2 *>(vb + c * S64_MEM + 32);
-            const double v[4] = {v01.x, v01.y, v23.x, v23.y};
+    };
+    set_tile((int)(s0 / pl.nkc), (int)(s0 % pl.nkc));
+
+    double cT[NT][4], cN[NT][4];
+    auto zero = [&]() {
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                double kT, kN = 0.0;
-                if (MODE == 2) {
-                    const double2 kk = *reinterpret_cast<const double2 *>(kb + i * KLD + 2 * c);
-                    kT = kk.x;
-                    kN = kk.y;
-                } else {
-                    kT = kb[i * KLD + c];
-                }
+        for (int n = 0; n < NT; n++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    aT[i][j] = fma(kT, v[j], aT[i][j]);
-                    if (MODE == 2) aN[i][j] = fma(kN, v[j], aN[i][j]);
-                }
-            }
-        }
-        __syncthreads();   // the buffer is refilled by the next iteration's copies
+            for (int j = 0; j < 4; j++) { cT[n][j] = 0.0; cN[n][j] = 0.0; }
+    };
+    zero();
+    const int nsteps = (int)(s1 - s0);
+#pragma unroll
+    for (int q = 0; q < ST - 1; q++) {
+        if (q < nsteps) load(q);
+        s64_commit();
     }
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const int64_t row = r0 + 2 * ty + i;
-        if (row >= N) continue;
+    int st = 0, tile = (int)(s0 / pl.nkc), c = (int)(s0 % pl.nkc);
+    for (int step = 0; step < nsteps; step++) {
+        s64_wait<ST - 2>();
+        __syncthreads();   // stage st is complete; the stage before it has been read by all
+        if (step + ST - 1 < nsteps) load(st == 0 ? ST - 1 : st - 1);
+        s64_commit();
+        const double *kb = s64_smem + st * STAGE + (16 * warp + g) * KLD;
+        const double *vb = s64_smem + st * STAGE + KSZ + g * S64_VROW + t4;
+        // one k step of 4 columns at a time over all members and components:
+        // consecutive instructions are independent (a k chain within one
+        // accumulator would wait for the unit's latency)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int m = m0 + (j < 2 ? 2 * tx + j : 32 + 2 * tx + (j - 2));
-            if (m >= R) continue;
-            const int64_t o = inst[m].poff + (int64_t)split * N + row;
-            partT[o] = aT[i][j];
-            if (MODE == 2) partN[o] = aN[i][j];
+            double aT[2], aN[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                if (MODE == 2) {
+                    const double2 kk = *reinterpret_cast<const double2 *>(kb + i * 8 * KLD + 2 * (t4 + 4 * j));
+                    aT[i] = kk.x;
+                    aN[i] = kk.y;
+                } else {
+                    aT[i] = kb[i * 8 * KLD + t4 + 4 * j];
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < NT; n++) {
+                const double b = vb[n * 8 * S64_VROW + 4 * j];
+                s64_mma(cT[n], aT, b);
+                if (MODE == 2) s64_mma(cN[n], aN, b);
+            }
+        }
+        st = st == ST - 1 ? 0 : st + 1;
+        const bool last = ++c == pl.nkc;
+        if (last || step + 1 == nsteps) {
+            // end of this CTA's piece of the tile
+            const int64_t b0 = s64_cta_of((int64_t)tile * pl.nkc, pl.steps, pl.ctas);
+            const int slot = (int)(blockIdx.x - b0);
+            const int64_t r0 = (int64_t)(tile / pl.mtiles) * S64_ROWS + 16 * warp + g;
+            const int m0 = tile % pl.mtiles * (8 * NT) + 2 * t4;
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const int64_t row = r0 + 8 * (j >> 1);
+                    const int m = m0 + 8 * n + (j & 1);
+                    if (row < N && m < R) {
+                        const int64_t o = inst[m].poff + row;
+                        partT[o + (int64_t)slot * N] = cT[n][j];
+                        if (MODE == 2) partN[o + (int64_t)slot * N] = cN[n][j];
+                        if (last)
+                            for (int q = slot + 1; q < pl.slots; q++) {
+                                partT[o + (int64_t)q * N] = 0.0;
+                                if (MODE == 2) partN[o + (int64_t)q * N] = 0.0;
+                            }
+                    }
+                }
+            zero();
+            tile++;
+            c = 0;
         }
     }
 }

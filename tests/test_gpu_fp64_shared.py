@@ -41,6 +41,27 @@ def test_fp64_shared_kv_matches_oracle(R, mode):
                 assert np.abs(gN[r] - oN).max() <= 1e-12 * np.abs(oN).max(), r
 
 
+@pytest.mark.parametrize("n_el,R", [(2, 3), (15, 8), (16, 9), (17, 56), (63, 57), (64, 129), (65, 64), (130, 256)])
+@pytest.mark.parametrize("mode", ["modeII", "modeIII"])
+def test_fp64_shared_tile_edges(n_el, R, mode):
+    """Rows around the 64-row tiles, columns around the 16-column chunks,
+    members around the 8-member tiles and the 64-member tiles."""
+    p = networks.single_fault(n_el=n_el, length=10.0 * n_el, mode=mode)
+    ps = networks.shared_geometry_ensemble(R, base=p, seed=1)
+    o = Oracle(p)
+    o.use_dense()
+    rng = np.random.default_rng(n_el)
+    with Ensemble(ps, storage="fp64_shared") as e:
+        slips = [rng.normal(0.0, 1.0, n_el) for _ in range(R)]
+        gT, gN = e.kernel(slips)
+        for r in range(R):
+            oT, oN = o.kernel(slips[r])
+            assert np.abs(gT[r] - oT).max() <= 1e-12 * np.abs(oT).max(), r
+            if mode == "modeII":
+                # a straight fault exerts no normal stress on itself: measured against the shear stress
+                assert np.abs(gN[r] - oN).max() <= 1e-12 * np.abs(oT).max(), r
+
+
 def test_fp64_shared_long_reduction_and_splits():
     """~2500 elements: 79 row tiles, 79 column chunks split over several
     CTAs; two calls in a row."""
