@@ -268,7 +268,10 @@ __global__ void assemble_kernel(int64_t N, int64_t Np, const double *__restrict_
 constexpr int GEMV_WARPS = 8;
 constexpr int GEMV_LPL = 8;                       // 16-byte loads per lane per row-chunk
 constexpr int GEMV_CHUNK_BYTES = 32 * GEMV_LPL * 16;  // 4096
-constexpr int GEMV_ROWS = 64;                     // rows per CTA
+// Rows per CTA where there are many waves of tiles. A tile's height is the
+// same for every tile of a handle, a multiple of the eight warps chosen by
+// gemv_rows(); heights change no sum.
+constexpr int GEMV_ROWS = 64;
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -347,7 +350,7 @@ __device__ __forceinline__ bool press_takes_part(const StepCtl *ctl, int i, int 
 // K.V streaming kernel (direct 128-bit loads).
 //
 // Work unit (tile): one 4 KiB column chunk of one instance for a block of
-// GEMV_ROWS rows. Every lane keeps the V values of its columns in registers
+// rows. Every lane keeps the V values of its columns in registers
 // and reuses them for all rows of the block; each warp owns rows r0+w,
 // r0+w+8, ... and issues 8 coalesced 128-bit loads per lane per row (two rows
 // in flight). The per-(chunk,row) warp sum goes to part[c*N + row]; the
@@ -371,7 +374,7 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32)
     double *pT = partT + I.poff, *pN = partN + I.poff;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t c = t.y;
-    const int64_t r0 = (int64_t)t.z * GEMV_ROWS;
+    const int64_t r0 = t.z, rend = r0 + t.w;
     const int64_t row_vecs = I.Np * BPC / 16;
 
     double v[GEMV_LPL * CPV];
@@ -384,9 +387,9 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32)
         }
 
     const int64_t vec0 = c * (CW * BPC / 16) + lane;
-    for (int64_t r = r0 + warp; r < r0 + GEMV_ROWS && r < N; r += 2 * GEMV_WARPS) {
+    for (int64_t r = r0 + warp; r < rend; r += 2 * GEMV_WARPS) {
         const int64_t rb = r + GEMV_WARPS;
-        const bool two = (rb < r0 + GEMV_ROWS) && (rb < N);
+        const bool two = rb < rend;
         const uint4 *pa = K + r * row_vecs + vec0;
         const uint4 *pb = K + (two ? rb : r) * row_vecs + vec0;
         uint4 qa[GEMV_LPL], qb[GEMV_LPL];
@@ -491,9 +494,8 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     double *pT = partT + I.poff, *pN = partN + I.poff;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t c = t.y;
-    const int64_t r0 = (int64_t)t.z * GEMV_ROWS;
-    const int64_t rend = (r0 + GEMV_ROWS < N) ? r0 + GEMV_ROWS : N;
-    const int nrows = (int)(rend - r0);
+    const int64_t r0 = t.z;
+    const int nrows = t.w;
     const int64_t row_bytes = I.Np * BPC;
 
     if (threadIdx.x == 0) {

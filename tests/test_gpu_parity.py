@@ -47,6 +47,22 @@ def test_kernel_matches_oracle(mode, storage, tol, gemv):
             assert rel(gN, oN) < tol
 
 
+@pytest.mark.parametrize("n_el", [2, 8, 9, 129, 1404, 2001, 2500])
+@pytest.mark.parametrize("mode,storage,tol", [("modeII", "fp64", 1e-12), ("modeIII", "fp64", 1e-12),
+                                              ("modeIII", "fp32", 2e-6), ("modeII", "bf16x2", 5e-5)])
+@pytest.mark.parametrize("gemv", ["tma", "ldg"])
+def test_kernel_tile_heights(n_el, mode, storage, tol, gemv):
+    """Tiles of 8 to 80 rows (the height follows the amount of work), last
+    tiles shorter than the others."""
+    p = networks.single_fault(n_el=n_el, length=10.0 * n_el, mode=mode)
+    o = Oracle(p, threads=8)
+    with Simulation(p, storage=storage, gemv=gemv) as s:
+        v = np.random.default_rng(n_el).normal(size=s.N)
+        gT, _ = s.kernel(v)
+        oT, _ = o.kernel(v)
+        assert rel(gT, oT) < tol * (10 if storage == "fp64" else 1)   # the matrix-free oracle: as below
+
+
 def test_kernel_large_single_fault_and_linearity():
     p = networks.single_fault(n_el=3000, length=30e3, mode="modeII")
     o = Oracle(p, threads=8)
