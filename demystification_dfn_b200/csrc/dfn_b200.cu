@@ -104,6 +104,7 @@ struct dfn_handle {
     int64_t nseg = 0, nseg0 = 0;
     int *long_seg = nullptr;              // segments longer than TRI_SHORT_MAX
     int64_t nlong = 0, nlong0 = 0;
+    int long_threads = TRI_NT1;           // threads that the longest of them takes
     int *short_seg = nullptr;             // the others
     int64_t nshort = 0, nshort0 = 0;
     int tri_shape = 0;                    // short segments: 0 a warp each, 1 a thread each, 2 tiles
@@ -528,7 +529,7 @@ static int launch_pressure(dfn_handle *h, int mask, int kind, int sys0, int nsys
         }
         if (nlong > 0) {
             dim3 lgrid((unsigned)nlong, (unsigned)nsys);
-            pressure_tridiag_long_kernel<<<lgrid, TRI_NT, 0, h->stream>>>(
+            pressure_tridiag_long_kernel<<<lgrid, h->long_threads, TRI_LONG_SMEM(h->long_threads), h->stream>>>(
                 h->pg, h->inst, h->ctl, mask, kind, sys0, dt_explicit, h->seg_start, h->seg_inst, h->long_seg,
                 h->Ptemp, h->Pdot_s, h->pwork);
         }
@@ -587,8 +588,11 @@ static ElemParams elem_params(dfn_handle *h)
 static cudaStream_t pressure_beside(dfn_handle *h, int nsys, int ninst)
 {
     if (!h->side_stream) return nullptr;
-    if (h->pressure == DFN_PRESSURE_TRIDIAG)
-        return (h->tc && h->tc_variant == 0 && h->tri_shape == 2 && h->nlong == 0) ? h->side_lo : nullptr;
+    if (h->pressure == DFN_PRESSURE_TRIDIAG) {
+        if (h->tc && h->tc_variant == 0 && h->tri_shape == 2 && h->nlong == 0) return h->side_lo;
+        // long segments alone, a CTA each
+        return (h->nshort == 0 && nsys * h->nlong <= h->sms / 2) ? h->side_stream : nullptr;
+    }
     if (h->pressure != DFN_PRESSURE_CG || h->pcl <= 0 || h->pcl_mode == 0 || h->pcl_mode == 2) return nullptr;
     if (h->pcl_mode < 0 && (int64_t)nsys * ninst > h->pcl_max) return nullptr;
     return ((int64_t)nsys * ninst * h->pcl <= h->sms / 2) ? h->side_stream : nullptr;
@@ -1711,6 +1715,7 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
         // those of network 0 come first
         std::vector<int> lg, sh;
         for (int64_t q = 0; q < h->nseg; q++) {
+            if (seg[q + 1] - seg[q] > TRI_NT1 * TRI_MAXM) h->long_threads = TRI_NT2;
             if (seg[q + 1] - seg[q] > TRI_SHORT_MAX) lg.push_back((int)q);
             else sh.push_back((int)q);
             if (q + 1 == h->nseg0) {
@@ -1745,6 +1750,8 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
             HCOPY(h->tri_tiles, tl.data(), tl.size());
         }
         if (h->nlong) {
+            CKC(cudaFuncSetAttribute(pressure_tridiag_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)TRI_LONG_SMEM(TRI_NT2)));
             DALLOC(h->long_seg, lg.size());
             HCOPY(h->long_seg, lg.data(), lg.size());
         }

@@ -669,6 +669,9 @@ __device__ __forceinline__ double pterms_x(const PressParams &p, int64_t k, doub
 __device__ __forceinline__ double psource(const PressParams &p, int64_t k, double dt)
 {
     double add = 0.0;
+    bool here = false;   // few elements have a source
+    for (int64_t j = 0; j < p.nsrc; j++) here |= p.src_elem[j] == k;
+    if (!here) return add;
     const double t = add_(*p.ctl_time, dt);
     for (int64_t s = 0; s < p.nsrc; s++) {
         if (!(t >= p.src_tb[s] && t < p.src_te[s])) continue;
@@ -740,13 +743,17 @@ __device__ __forceinline__ void block_sum_max(double a, double b, double *red, d
 }
 
 // Segments of at most TRI_SHORT_MAX elements are solved by one warp each
-// (pressure_tridiag_kernel, up to TRI_WMAXM rows per lane), longer ones by a
-// CTA of TRI_NT threads (pressure_tridiag_long_kernel), rows in registers up
-// to TRI_MAXM rows per thread.
+// (pressure_tridiag_kernel, up to TRI_WMAXM rows per lane), longer ones by
+// TRI_NT1 threads of a CTA, or TRI_NT2 beyond TRI_NT1 * TRI_MAXM elements
+// (pressure_tridiag_long_kernel), rows in registers up to TRI_MAXM rows per
+// thread. The threads that a segment gets depend on its length alone, so its
+// results do not depend on what else is in the launch.
 #define TRI_SHORT_MAX 64
 #define TRI_WMAXM 2
-#define TRI_NT 256
-#define TRI_MAXM 16
+#define TRI_NT1 256
+#define TRI_NT2 1024
+#define TRI_MAXM 4
+#define TRI_LONG_SMEM(nt) (sizeof(double) * 4 * TRI_MAXM * (nt))
 
 // System s of a pressure launch gets its dt from the controller:
 //   kind 0: dt = ctl->t_try (probe / first RHS), halving on non-convergence
@@ -824,6 +831,9 @@ __device__ __forceinline__ double pmatvec_row_s(int64_t k, int64_t N, double s1,
 __device__ __forceinline__ double pb1(const PressParams &p, int64_t k, double dt, double diag)
 {
     double b1 = __ddiv_rn(p.P[k], diag);
+    bool here = false;   // few elements have a source
+    for (int64_t j = 0; j < p.nsrc; j++) here |= p.src_elem[j] == k;
+    if (!here) return b1;
     const double t = add_(*p.ctl_time, dt);
     for (int64_t s = 0; s < p.nsrc; s++) {
         if (!(t >= p.src_tb[s] && t < p.src_te[s])) continue;
@@ -1424,35 +1434,46 @@ __device__ __forceinline__ Aff shfl_down(const Aff &v, int d)
     return {__shfl_down_sync(0xffffffffu, v.a, d), __shfl_down_sync(0xffffffffu, v.b, d)};
 }
 
+// Barrier of the first NTG threads of the CTA (the others have left).
+template <int NTG>
+__device__ __forceinline__ void grp_sync()
+{
+    asm volatile("bar.sync 1, %0;" ::"n"(NTG) : "memory");
+}
+
 // Exclusive forward scan over the group (thread 0 first): returns the
-// composition of the maps of threads 0..t-1 (identity for t = 0).
+// composition of the maps of threads 0..t-1 (identity for t = 0). Warps by
+// shuffles, then warp 0 scans the warps' totals the same way.
 template <int NTG, typename T>
 __device__ __forceinline__ T grp_scan_excl(T v, T ident, T *sm)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = NTG / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int NW = NTG / 32;
+#pragma unroll 1
     for (int d = 1; d < 32; d <<= 1) {
         T o = shfl_up(v, d);
         if (lane >= d) v = compose(v, o);
     }
-    if constexpr (NTG == 32) {
-        T prev = shfl_up(v, 1);
-        return (lane == 0) ? ident : prev;
-    }
-    __syncthreads();
-    if (lane == 31) sm[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        T acc = ident;
-        for (int q = 0; q < nw; q++) {
-            T tot = sm[q];
-            sm[q] = acc;               // prefix of the warps before q
-            acc = compose(tot, acc);
-        }
-    }
-    __syncthreads();
     T prev = shfl_up(v, 1);
-    const T wp = sm[w];
-    return (lane == 0) ? wp : compose(prev, wp);
+    if (lane == 0) prev = ident;
+    if constexpr (NTG > 32) {
+        grp_sync<NTG>();
+        if (lane == 31) sm[w] = v;
+        grp_sync<NTG>();
+        if (w == 0) {
+            T t = lane < NW ? sm[lane] : ident;
+#pragma unroll 1
+            for (int d = 1; d < NW; d <<= 1) {
+                T o = shfl_up(t, d);
+                if (lane >= d) t = compose(t, o);
+            }
+            t = shfl_up(t, 1);
+            if (lane < NW) sm[lane] = lane == 0 ? ident : t;
+        }
+        grp_sync<NTG>();
+        prev = compose(prev, sm[w]);
+    }
+    return prev;
 }
 
 // Exclusive backward scan for affine maps: the composition of the maps of
@@ -1460,66 +1481,76 @@ __device__ __forceinline__ T grp_scan_excl(T v, T ident, T *sm)
 template <int NTG>
 __device__ __forceinline__ Aff grp_scan_excl_back(Aff v, Aff *sm)
 {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = NTG / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int NW = NTG / 32;
+#pragma unroll 1
     for (int d = 1; d < 32; d <<= 1) {
         Aff o = shfl_down(v, d);
         if (lane + d < 32) v = compose(v, o);
     }
-    if constexpr (NTG == 32) {
-        Aff next = shfl_down(v, 1);
-        return (lane == 31) ? aff_id() : next;
-    }
-    __syncthreads();
-    if (lane == 0) sm[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        Aff acc = aff_id();
-        for (int q = nw - 1; q >= 0; q--) {
-            Aff tot = sm[q];
-            sm[q] = acc;               // composition of the warps after q
-            acc = compose(tot, acc);
-        }
-    }
-    __syncthreads();
     Aff next = shfl_down(v, 1);
-    const Aff ws = sm[w];
-    return (lane == 31) ? ws : compose(next, ws);
+    if (lane == 31) next = aff_id();
+    if constexpr (NTG > 32) {
+        grp_sync<NTG>();
+        if (lane == 0) sm[w] = v;
+        grp_sync<NTG>();
+        if (w == 0) {
+            Aff t = lane < NW ? sm[lane] : aff_id();
+#pragma unroll 1
+            for (int d = 1; d < NW; d <<= 1) {
+                Aff o = shfl_down(t, d);
+                if (lane + d < NW) t = compose(t, o);
+            }
+            t = shfl_down(t, 1);
+            if (lane < NW) sm[lane] = lane == NW - 1 ? aff_id() : t;
+        }
+        grp_sync<NTG>();
+        next = compose(next, sm[w]);
+    }
+    return next;
 }
 
 // f(j) for the rows j < nr of this thread, in order (REV: reverse order);
-// with MAXM > 0 the loop is unrolled so that register arrays stay registers.
-template <int MAXM, bool REV, typename F>
+// with UNROLL > 0 unrolled so that register arrays stay registers.
+template <int UNROLL, bool REV, typename F>
 __device__ __forceinline__ void tri_rows(int nr, F f)
 {
-    if constexpr (MAXM > 0) {
+    if constexpr (UNROLL > 0) {
 #pragma unroll
-        for (int q = 0; q < MAXM; q++) {
-            const int j = REV ? MAXM - 1 - q : q;
+        for (int q = 0; q < UNROLL; q++) {
+            const int j = REV ? UNROLL - 1 - q : q;
             if (j < nr) f(j);
         }
     } else {
+#pragma unroll 1
         for (int q = 0; q < nr; q++) f(REV ? nr - 1 - q : q);
     }
 }
 
+// Rows of a thread live in registers (a warp), in shared memory (sm: 4 x MAXM
+// x NTG doubles) or, MAXM = 0, in the global work area gw.
 template <int NTG, int MAXM>
 __device__ __forceinline__ void tri_segment(const PressParams &p, double dt, int64_t k0, int64_t k1, double *Pt,
-                                            double *Pd, double *gw, int64_t N, Mob *smm, Aff *sma, int &bad)
+                                            double *Pd, double *gw, double *sm, int64_t N, Mob *smm, Aff *sma,
+                                            int &bad)
 {
     const int64_t L = k1 - k0;
     const int tid = (NTG == 32) ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
     const int64_t m = (L + NTG - 1) / NTG;
     const int64_t r0 = (int64_t)tid * m;
     const int nr = (int)max((int64_t)0, min(m, L - r0));
-    constexpr int R = (MAXM > 0) ? MAXM : 1;
+    constexpr bool REGS = NTG == 32;
+    constexpr int UNROLL = REGS ? MAXM : 0;
+    constexpr int R = REGS ? MAXM : 1;
     double reg[4][R];
     // row q of element j of this thread: A1, 1/den (A2 on input), c (A3 on
     // input), d (right-hand side on input)
     auto at = [&](int q, int j) -> double & {
-        if constexpr (MAXM > 0) return reg[q][j];
+        if constexpr (REGS) return reg[q][j];
+        else if constexpr (MAXM > 0) return sm[(q * MAXM + j) * NTG + tid];
         else return gw[(int64_t)q * N + k0 + r0 + j];
     };
-    tri_rows<MAXM, false>(nr, [&](int j) {
+    tri_rows<UNROLL, false>(nr, [&](int j) {
         const int64_t k = k0 + r0 + j;
         double A1, A2, A3;
         prow_tri(p, k, dt, A1, A2, A3);
@@ -1530,28 +1561,28 @@ __device__ __forceinline__ void tri_segment(const PressParams &p, double dt, int
     });
     // c recurrence
     Mob T = mob_id();
-    tri_rows<MAXM, false>(nr, [&](int j) { T = compose(Mob{0.0, at(2, j), -at(0, j), at(1, j)}, T); });
+    tri_rows<UNROLL, false>(nr, [&](int j) { T = compose(Mob{0.0, at(2, j), -at(0, j), at(1, j)}, T); });
     const Mob E = grp_scan_excl<NTG>(T, mob_id(), smm);
     double c = (tid == 0) ? 0.0 : E.b / E.d;
-    tri_rows<MAXM, false>(nr, [&](int j) {
+    tri_rows<UNROLL, false>(nr, [&](int j) {
         const double rden = 1.0 / (at(1, j) - at(0, j) * c);
         c = at(2, j) * rden;
         at(1, j) = rden; at(2, j) = c;
     });
     // d recurrence
     Aff F = aff_id();
-    tri_rows<MAXM, false>(nr, [&](int j) { F = compose(Aff{-at(0, j) * at(1, j), at(3, j) * at(1, j)}, F); });
+    tri_rows<UNROLL, false>(nr, [&](int j) { F = compose(Aff{-at(0, j) * at(1, j), at(3, j) * at(1, j)}, F); });
     double d = grp_scan_excl<NTG>(F, aff_id(), sma).b;
-    tri_rows<MAXM, false>(nr, [&](int j) {
+    tri_rows<UNROLL, false>(nr, [&](int j) {
         d = (at(3, j) - at(0, j) * d) * at(1, j);
         at(3, j) = d;
     });
     // back substitution
     Aff G = aff_id();
-    tri_rows<MAXM, true>(nr, [&](int j) { G = compose(Aff{-at(2, j), at(3, j)}, G); });
+    tri_rows<UNROLL, true>(nr, [&](int j) { G = compose(Aff{-at(2, j), at(3, j)}, G); });
     double x = grp_scan_excl_back<NTG>(G, sma).b;
     const double rdt = (dt < 1e-9) ? 0.0 : 1.0 / dt;
-    tri_rows<MAXM, true>(nr, [&](int j) {
+    tri_rows<UNROLL, true>(nr, [&](int j) {
         const int64_t k = k0 + r0 + j;
         x = at(3, j) - at(2, j) * x;
         Pt[k] = x;
@@ -1738,21 +1769,26 @@ __global__ void __launch_bounds__(256) pressure_tridiag_kernel(PressGlobal g, co
     const int64_t k0 = seg_start[sg] - I.eoff, k1 = seg_start[sg + 1] - I.eoff;
     double *Pt = Ptemp + 6 * I.eoff + (int64_t)sys * N, *Pd = Pdot + 6 * I.eoff + (int64_t)sys * N;
     int bad = 0;
-    tri_segment<32, TRI_WMAXM>(p, dt, k0, k1, Pt, Pd, nullptr, N, nullptr, nullptr, bad);
+    tri_segment<32, TRI_WMAXM>(p, dt, k0, k1, Pt, Pd, nullptr, nullptr, N, nullptr, nullptr, bad);
     if (bad) atomicCAS(&ctl[i].status, 0, 4);
 }
 
-// grid (long segments of the launch, systems); blockDim = TRI_NT.
-__global__ void __launch_bounds__(TRI_NT, 1) pressure_tridiag_long_kernel(PressGlobal g, const Inst *inst,
-                                                                          StepCtl *ctl, int mask, int kind, int sys0,
-                                                                          double dt_explicit,
-                                                                          const int64_t *seg_start,
-                                                                          const int *seg_inst, const int *long_seg,
-                                                                          double *Ptemp, double *Pdot, double *work)
+// grid (long segments of the launch, systems); blockDim = TRI_NT2 when the
+// handle has segments longer than TRI_NT1 * TRI_MAXM, else TRI_NT1. The solve
+// is a chain of latencies (serial rows, three scans), so few rows per thread,
+// scans over the warps' totals, and rolled loops over rows in shared memory
+// (unrolled, the code is fetched once per launch and the fetch dominates): 4000 elements on 256 threads of 16 rows,
+// one thread adding up the warps, took 58 us, now 25 (cold caches).
+__global__ void __launch_bounds__(TRI_NT2, 1) pressure_tridiag_long_kernel(PressGlobal g, const Inst *inst,
+                                                                           StepCtl *ctl, int mask, int kind, int sys0,
+                                                                           double dt_explicit,
+                                                                           const int64_t *seg_start,
+                                                                           const int *seg_inst, const int *long_seg,
+                                                                           double *Ptemp, double *Pdot, double *work)
 {
-    __shared__ Mob smm[TRI_NT / 32];
-    __shared__ Aff sma[TRI_NT / 32];
-    __shared__ int sbad;
+    extern __shared__ __align__(16) double tri_sm[];
+    __shared__ Mob smm[TRI_NT2 / 32];
+    __shared__ Aff sma[TRI_NT2 / 32];
     const int sg = long_seg[blockIdx.x];
     const int i = seg_inst[sg];
     if (!press_takes_part(ctl, i, mask, kind)) return;       // uniform over the CTA
@@ -1764,15 +1800,16 @@ __global__ void __launch_bounds__(TRI_NT, 1) pressure_tridiag_long_kernel(PressG
     const int64_t k0 = seg_start[sg] - I.eoff, k1 = seg_start[sg + 1] - I.eoff;
     double *Pt = Ptemp + 6 * I.eoff + (int64_t)sys * N, *Pd = Pdot + 6 * I.eoff + (int64_t)sys * N;
     double *gw = work + 24 * I.eoff + (int64_t)sys * 4 * N;
-    if (threadIdx.x == 0) sbad = 0;
     int bad = 0;
-    if (k1 - k0 <= (int64_t)TRI_NT * TRI_MAXM)
-        tri_segment<TRI_NT, TRI_MAXM>(p, dt, k0, k1, Pt, Pd, gw, N, smm, sma, bad);
-    else
-        tri_segment<TRI_NT, 0>(p, dt, k0, k1, Pt, Pd, gw, N, smm, sma, bad);
-    if (bad) atomicOr(&sbad, 1);
-    __syncthreads();
-    if (threadIdx.x == 0 && sbad) atomicCAS(&ctl[i].status, 0, 4);
+    if (k1 - k0 <= (int64_t)TRI_NT1 * TRI_MAXM) {
+        if (threadIdx.x >= TRI_NT1) return;
+        tri_segment<TRI_NT1, TRI_MAXM>(p, dt, k0, k1, Pt, Pd, gw, tri_sm, N, smm, sma, bad);
+    } else if (k1 - k0 <= (int64_t)TRI_NT2 * TRI_MAXM) {
+        tri_segment<TRI_NT2, TRI_MAXM>(p, dt, k0, k1, Pt, Pd, gw, tri_sm, N, smm, sma, bad);
+    } else {
+        tri_segment<TRI_NT2, 0>(p, dt, k0, k1, Pt, Pd, gw, tri_sm, N, smm, sma, bad);
+    }
+    if (bad) atomicCAS(&ctl[i].status, 0, 4);
 }
 
 // ---------------------------------------------------------------------------

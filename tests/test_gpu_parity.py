@@ -110,6 +110,19 @@ def _cluster_case(case):
 
 
 @pytest.mark.parametrize("case", ["single4000", "net300", "net500"])
+@pytest.mark.parametrize("n_el", [65, 256, 257, 1023, 1024, 1025, 2047, 4096, 4097, 6000])
+def test_long_tridiagonal_segments(n_el):
+    """One fault longer than a warp's segment: 256 threads, 1024 threads and
+    the global-memory rows, full and partly filled groups."""
+    p = networks.single_fault(n_el=n_el, length=10.0 * n_el, mode="modeIII", tol=1e-6)
+    o = Oracle(p)
+    with Simulation(p, storage="fp32", pressure="tridiag") as s:
+        for dt in (1.0, 5e4):
+            gP, _, _ = s.compute_P(dt)
+            ex = o.pressure_exact(dt)
+            assert np.abs(gP - ex).max() <= 1e-12 * np.abs(ex).max()
+
+
 @pytest.mark.parametrize("dt", [10.0, 3600.0, 86400.0])
 @pytest.mark.parametrize("form", ["cluster", "cta_smem", "cta"])
 def test_pressure_cg_cluster_matches_oracle(case, dt, form):
