@@ -131,6 +131,7 @@ struct dfn_handle {
     bool pcoup = false;
     double *kstar = nullptr, *kmin = nullptr, *Snk = nullptr;
     int *err_flag = nullptr;
+    unsigned int *ticket = nullptr;       // blocks of the round's last launch that are done
     int wait_polls = MBAR_POLLS;          // polls of the TMA K.V pipeline's bounded waits
     void *K = nullptr;
     size_t K_bytes = 0;
@@ -610,13 +611,10 @@ static int launch_pressure_side(dfn_handle *h, cudaStream_t side, int mask, int 
     return DFN_OK;
 }
 
-// One RK attempt (stages 2..6 and the error test) of every network in `mask`.
-static int run_attempt(dfn_handle *h, int mask)
+// Stages 2..6 of an RK attempt of every network in `mask`, from the ytemp of
+// stage 2.
+static int run_stages(dfn_handle *h, int mask)
 {
-    attempt_begin_kernel<<<blocks_of(h->Ntot, 256), 256, 0, h->stream>>>(elem_params(h), h->Y, h->kbuf, h->ytmp,
-                                                                         mask);
-    h->launches++;
-    CKL();
     // the Newton formulation interpolates the stage pressure in time and
     // needs only the full-step system (c = 1)
     const int sys0 = h->form == DFN_FORM_NEWTON ? 4 : 1, nsys = h->form == DFN_FORM_NEWTON ? 1 : 5;
@@ -631,10 +629,27 @@ static int run_attempt(dfn_handle *h, int mask)
         if (s == 2 && beside) CK(cudaStreamWaitEvent(h->stream, h->ev_pjoin, 0));
         TRY(launch_friction(h, s, s - 1, mask, h->Ntot));
     }
+    return DFN_OK;
+}
+
+// Step control of the networks in `mask` by itself.
+static int run_decide(dfn_handle *h, int mask)
+{
     decide_kernel<<<blocks_of(h->B, 128), 128, 0, h->stream>>>(h->ctl, h->B, mask);
     h->launches++;
     CKL();
     return DFN_OK;
+}
+
+// One RK attempt (stages 2..6 and the error test) of every network in `mask`.
+static int run_attempt(dfn_handle *h, int mask)
+{
+    attempt_begin_kernel<<<blocks_of(h->Ntot, 256), 256, 0, h->stream>>>(elem_params(h), h->Y, h->kbuf, h->ytmp,
+                                                                         mask);
+    h->launches++;
+    CKL();
+    TRY(run_stages(h, mask));
+    return run_decide(h, mask);
 }
 
 // Permeability coupling: the permeability and face values of the networks
@@ -656,13 +671,10 @@ static int perm_refresh(dfn_handle *h, int mask, int accepted_only)
     return DFN_OK;
 }
 
-// One round of the solve() loop for every network of the batch.
+// One round of the solve() loop for every network of the batch (the
+// controllers stand at the start of a step or of a further attempt).
 static int run_round(dfn_handle *h)
 {
-    const unsigned bb = blocks_of(h->B, 128);
-    step_begin_kernel<<<bb, 128, 0, h->stream>>>(h->ctl, h->inst, h->B, h->src_tb);
-    h->launches++;
-    CKL();
     // coupled permeability of a new step: from sigmaN and P committed
     if (h->pcoup) TRY(perm_refresh(h, M_NEW, 0));
     // CG probe at t_try (halving on non-convergence); its solution is the
@@ -676,13 +688,12 @@ static int run_round(dfn_handle *h)
     if (after) TRY(launch_pressure_side(h, side, M_NEW, 0, 0, 1, h->B));
     if (beside) CK(cudaStreamWaitEvent(h->stream, h->ev_pjoin, 0));
     TRY(launch_friction(h, 1, 0, M_NEW, h->Ntot));
-    set_h_kernel<<<bb, 128, 0, h->stream>>>(h->ctl, h->B);
-    h->launches++;
-    CKL();
-    TRY(run_attempt(h, M_ACTIVE));
-    commit_kernel<<<blocks_of(h->Ntot, 256), 256, 0, h->stream>>>(
+    TRY(run_stages(h, M_ACTIVE));
+    if (h->pcoup) TRY(run_decide(h, M_ACTIVE));
+    (h->pcoup ? commit_kernel<false> : commit_kernel<true>)<<<blocks_of(h->Ntot, 256), 256, 0, h->stream>>>(
         elem_params(h), h->Y, h->yout, h->P, h->Pdot, h->Ptemp, h->Pdot_s,
-        h->form == DFN_FORM_NEWTON ? nullptr : h->slip, h->slip_out, h->pcoup ? 0 : 1);
+        h->form == DFN_FORM_NEWTON ? nullptr : h->slip, h->slip_out, h->kbuf, h->ytmp, h->pcoup ? 0 : 1, h->B,
+        h->src_tb, h->max_step, h->ticket);
     h->launches++;
     CKL();
     if (h->pcoup) {
@@ -695,10 +706,10 @@ static int run_round(dfn_handle *h)
                                                                         h->Pdot_s);
         h->launches++;
         CKL();
+        finish_kernel<<<blocks_of(h->B, 128), 128, 0, h->stream>>>(h->ctl, h->inst, h->B, h->src_tb, h->max_step);
+        h->launches++;
+        CKL();
     }
-    finish_kernel<<<bb, 128, 0, h->stream>>>(h->ctl, h->B, h->max_step);
-    h->launches++;
-    CKL();
     return DFN_OK;
 }
 
@@ -785,8 +796,8 @@ static int run_rounds(dfn_handle *h, int64_t n)
 
 static int solve_impl(dfn_handle *h, int64_t nsteps, double t_end)
 {
-    arm_kernel<<<blocks_of(h->B, 128), 128, 0, h->stream>>>(h->ctl, h->B, (long long)nsteps, t_end,
-                                                            h->max_attempts);
+    arm_kernel<<<blocks_of(h->B, 128), 128, 0, h->stream>>>(h->ctl, h->inst, h->B, h->src_tb, (long long)nsteps,
+                                                            t_end, h->max_attempts);
     h->launches++;
     CKL();
     int64_t group = (t_end > 0.0) ? 8 : std::max<int64_t>(nsteps, 1);
@@ -1356,7 +1367,7 @@ int32_t dfn_destroy(dfn_handle *h)
                     h->nrm, h->permx, h->a, h->b, h->Dc, h->f0, h->V0, h->nload, h->sload, h->perm, h->fake,
                     h->src_fault, h->src_elem, h->src_Q, h->src_tb, h->src_te, h->Y, h->P, h->Pdot, h->yout,
                     h->yscal, h->ytmp, h->kbuf, h->SigT, h->SigN, h->partT, h->partN, h->Ptemp, h->Pdot_s,
-                    h->pwork, h->pcoef, h->vin, h->vout, h->snap, h->err_flag, h->K, h->ctl};
+                    h->pwork, h->pcoef, h->vin, h->vout, h->snap, h->err_flag, h->ticket, h->K, h->ctl};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
@@ -1607,12 +1618,13 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
     DALLOC(h->Ptemp, 6 * Nt); DALLOC(h->Pdot_s, 6 * Nt); DALLOC(h->pwork, 24 * Nt);
     if (h->pressure != DFN_PRESSURE_TRIDIAG) DALLOC(h->pcoef, 18 * Nt);
     DALLOC(h->vin, 3 * h->hinst[0].N); DALLOC(h->vout, 3 * h->hinst[0].N); DALLOC(h->snap, 5 * Nt);
-    DALLOC(h->err_flag, 1); DALLOC(h->ctl, count);
+    DALLOC(h->err_flag, 1); DALLOC(h->ticket, 1); DALLOC(h->ctl, count);
     DALLOC(h->slip, Nt); DALLOC(h->slip_out, Nt); DALLOC(h->slip_acc, Nt);
     CKC(cudaMemsetAsync(h->slip, 0, sizeof(double) * Nt, h->stream));
     DALLOC(h->src_fault, soff); DALLOC(h->src_elem, soff); DALLOC(h->src_Q, soff); DALLOC(h->src_tb, soff);
     DALLOC(h->src_te, soff);
     CKC(cudaMemsetAsync(h->err_flag, 0, sizeof(int), h->stream));
+    CKC(cudaMemsetAsync(h->ticket, 0, sizeof(unsigned int), h->stream));
     CKC(cudaMemsetAsync(h->partN, 0, sizeof(double) * std::max<int64_t>(poff, 1), h->stream));
     CKC(cudaMemsetAsync(h->Pdot, 0, sizeof(double) * Nt, h->stream));
     CKC(cudaMemsetAsync(h->SigT, 0, sizeof(double) * Nt, h->stream));

@@ -1978,7 +1978,7 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long *addr, double 
 }
 
 // stage: 0 = standalone evaluation (ytmp in, kbuf slot 0 out)
-//        1 = k1 at the step start (y in), also yscal
+//        1 = k1 at the step start (y in), also yscal, ytemp of stage 2 and the attempt's step
 //        2..5 = k_s, then ytemp of stage s+1 in place
 //        6 = k6, then yout, yerr and the max-norm contribution
 // sys: pressure system of this evaluation; mask: phases that take part.
@@ -2084,6 +2084,10 @@ __global__ void __launch_bounds__(128, LEARNED ? 5 : 8) friction_kernel(FricPara
             ysc[k] = add_(add_(fabs(yi[k]), fabs(mul_(dV, tt))), tol);
             ysc[N + k] = add_(add_(fabs(yi[N + k]), fabs(mul_(dpsi, tt))), tol);
             ysc[2 * N + k] = add_(add_(fabs(yi[2 * N + k]), fabs(mul_(dsig, tt))), tol);
+            // the first attempt's step is t_try: ytemp of stage 2
+#pragma unroll
+            for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(2, tt, yi[j * N + k], kb, S, j * N + k);
+            if (k == 0) ctl->h = tt;   // read by later launches only
         } else if (stage >= 2 && stage <= 5) {
             const double h = ctl->h;
 #pragma unroll
@@ -2181,6 +2185,8 @@ __global__ void newton_init_kernel(int64_t Ntot, const int *inst_of, const Inst 
     y[k] = 0.0;
 }
 
+__device__ __forceinline__ void ctl_attempt_begin(StepCtl &c);
+
 // Element-wise kernels over all instances; k == 0 of an instance also
 // updates that instance's scalars.
 struct ElemParams {
@@ -2190,7 +2196,8 @@ struct ElemParams {
     StepCtl *ctl;
 };
 
-// ytemp of stage 2 at the start of every attempt (h may have changed).
+// ytemp of stage 2 at the start of an attempt (dfn_rkqs; in the solve loop
+// the first stage and the end of a round form it).
 __global__ void attempt_begin_kernel(ElemParams ep, const double *y, const double *kbuf, double *ytmp, int mask)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -2204,47 +2211,62 @@ __global__ void attempt_begin_kernel(ElemParams ep, const double *y, const doubl
     double *yt = ytmp + 3 * I.eoff;
 #pragma unroll
     for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(2, h, yi[j * N + k], kb, 3 * N, j * N + k);
-    if (k == 0) {
-        ep.ctl[i].errmax_bits = 0ull;
-        ep.ctl[i].pfail_mask = 0;
-        ep.ctl[i].attempts += 1;
-    }
+    if (k == 0) ctl_attempt_begin(ep.ctl[i]);
 }
 
-// Step control after an attempt, one thread per instance:
-// src/ode_solver/ode_bs.f90:158-172.
+// The decision on an attempt from its error norm: src/ode_solver/
+// ode_bs.f90:158-172. Reads the controller only, so that every thread of a
+// launch can take it before the controller moves on.
+struct Decision {
+    bool accept;
+    double errmax, h;   // h: the step of the next attempt when rejected
+};
+__device__ __forceinline__ Decision decide(const StepCtl &c)
+{
+    const double SAFETY = 0.9, PSHRNK = -0.25;
+    Decision d;
+    d.errmax = __longlong_as_double((long long)c.errmax_bits) / c.eps;
+    d.accept = d.errmax <= 1.0;
+    d.h = c.h;
+    if (!d.accept) d.h = copysign(fmax(fabs(SAFETY * c.h * pow(d.errmax, PSHRNK)), 0.1 * fabs(c.h)), c.h);
+    return d;
+}
+__device__ __forceinline__ void ctl_decide(StepCtl &c, const Decision &d)
+{
+    const double SAFETY = 0.9, PGROW = -0.2;
+    const double ERRCON = (double)1.89e-4f;  // default-real literal in the reference
+    c.step_attempts += 1;
+    c.accepted = d.accept ? 1 : 0;
+    if (d.accept) {
+        c.hnext = (d.errmax > ERRCON) ? SAFETY * c.h * pow(d.errmax, PGROW) : 5.0 * c.h;
+        c.hdid = c.h;
+    } else {
+        c.rejected += 1;
+        c.h = d.h;
+        if (c.x + c.h == c.x) atomicCAS(&c.status, 0, 2);
+        else if (c.step_attempts >= c.max_attempts) atomicCAS(&c.status, 0, 8);
+    }
+}
+__device__ __forceinline__ void ctl_attempt_begin(StepCtl &c)
+{
+    c.errmax_bits = 0ull;
+    c.pfail_mask = 0;
+    c.attempts += 1;
+}
+
+// Step control after an attempt, one thread per instance (dfn_rkqs and runs
+// with permeability coupling).
 __global__ void decide_kernel(StepCtl *ctl, int B, int mask)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B || !takes_part(ctl, i, mask)) return;
-    StepCtl &c = ctl[i];
-    const double SAFETY = 0.9, PGROW = -0.2, PSHRNK = -0.25;
-    const double ERRCON = (double)1.89e-4f;  // default-real literal in the reference
-    double errmax = __longlong_as_double((long long)c.errmax_bits) / c.eps;
-    double h = c.h;
-    c.step_attempts += 1;
-    if (errmax <= 1.0) {
-        c.accepted = 1;
-        c.hnext = (errmax > ERRCON) ? SAFETY * h * pow(errmax, PGROW) : 5.0 * h;
-        c.hdid = h;
-    } else {
-        c.accepted = 0;
-        c.rejected += 1;
-        double htemp = SAFETY * h * pow(errmax, PSHRNK);
-        h = copysign(fmax(fabs(htemp), 0.1 * fabs(h)), h);
-        c.h = h;
-        if (c.x + h == c.x) atomicCAS(&c.status, 0, 2);
-        else if (c.step_attempts >= c.max_attempts) atomicCAS(&c.status, 0, 8);
-    }
+    ctl_decide(ctl[i], decide(ctl[i]));
 }
 
-// Start of one pass of solve() for instances beginning a step:
+// Start of one pass of solve() for an instance beginning a step:
 // src/solver.f90:60-77.
-__global__ void step_begin_kernel(StepCtl *ctl, const Inst *inst, int B, const double *src_tb)
+__device__ __forceinline__ void ctl_step_begin(StepCtl &c, const Inst &I, const double *src_tb)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B || ctl[i].phase != PH_NEW) return;
-    StepCtl &c = ctl[i];
     c.it_count += 1;
     c.accepted = 0;
     c.probe_ier = 0;
@@ -2252,7 +2274,6 @@ __global__ void step_begin_kernel(StepCtl *ctl, const Inst *inst, int B, const d
     c.commit_bad = 0;
     c.x = 0.0;
     if (c.t_try > 10.0) {
-        const Inst &I = inst[i];
         for (int64_t s = 0; s < I.nsrc; s++) {
             const double tb = src_tb[I.soff + s];
             if (c.time < tb && c.time + c.t_try > tb) c.t_try = 10.0;
@@ -2263,11 +2284,40 @@ __global__ void step_begin_kernel(StepCtl *ctl, const Inst *inst, int B, const d
     if (c.t_end > 0.0 && c.time + c.t_try > c.t_end) c.t_try = c.t_end - c.time;
 }
 
-__global__ void set_h_kernel(StepCtl *ctl, int B)
+// End of one pass of solve() for an instance (src/solver.f90:117-196): time,
+// t_try with the 1-day cap, the stop rules on the committed state
+// (check_errors, src/solver.f90:412-418; non-finite values too), the
+// instance's next phase, and the start of its next step or attempt.
+__device__ __forceinline__ void ctl_finish(StepCtl &c, const Inst &I, const double *src_tb, double t_cap)
+{
+    if (c.status != 0) {
+        c.phase = PH_DONE;
+    } else if (!c.accepted) {
+        c.phase = PH_RETRY;
+    } else {
+        c.time = c.time + c.hdid;
+        double tn = c.hnext;
+        if (tn > t_cap) tn = t_cap;
+        c.t_try = tn;
+        c.steps_done += 1;
+        if (c.commit_bad) {
+            c.status = (c.commit_bad & 1) ? 3 : 4;
+            c.phase = PH_DONE;
+        } else {
+            const bool done = (c.steps_done >= c.target_steps) ||
+                              (c.t_end > 0.0 && c.time >= c.t_end * (1.0 - 1e-14));
+            c.phase = done ? PH_DONE : PH_NEW;
+        }
+    }
+    if (c.phase == PH_NEW) ctl_step_begin(c, I, src_tb);
+    if (c.phase != PH_DONE) ctl_attempt_begin(c);
+}
+
+__global__ void finish_kernel(StepCtl *ctl, const Inst *inst, int B, const double *src_tb, double t_cap)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B || ctl[i].phase != PH_NEW) return;
-    ctl[i].h = ctl[i].t_try;
+    if (i >= B || !takes_part(ctl, i, M_ACTIVE)) return;
+    ctl_finish(ctl[i], inst[i], src_tb, t_cap);
 }
 
 // ---------------------------------------------------------------------------
@@ -2330,68 +2380,87 @@ __global__ void commit_p_kernel(ElemParams ep, double *P, double *Pdot, const do
     Pdot[e] = Pdot_s[6 * I.eoff + 5 * N + k];
 }
 
-// Accepted attempts: Y = yout, and the pressure commit compute_P(t_did),
-// which equals the stage-5 solve of the accepted attempt (dt = 0 + 1.0*h).
-// The whole state is committed before the stop rules look at it, as the
-// reference commits Y, P and time before check_errors (src/solver.f90:
-// 170-197): an extensional or non-finite component only raises a flag here,
-// which finish_kernel turns into the status after the time update.
+// End of a round. Accepted attempts: Y = yout, and the pressure commit
+// compute_P(t_did), which equals the stage-5 solve of the accepted attempt
+// (dt = 0 + 1.0*h). The whole state is committed before the stop rules look
+// at it, as the reference commits Y, P and time before check_errors
+// (src/solver.f90:170-197): an extensional or non-finite component only
+// raises a flag here, which ctl_finish turns into the status after the time
+// update. Rejected attempts: ytemp of stage 2 for the next attempt's step.
+// FUSED: the decision is taken here by every thread from the controllers as
+// the attempt left them, and the last block to finish moves the controllers
+// on (decision, end of the step, start of the next one): one launch where
+// there were six (ytemp, step sizes, decision, commit, finish, step start),
+// which cost 2.3 to 5 us each and are all latency. Otherwise decide_kernel
+// has run before and finish_kernel follows (permeability coupling solves the
+// pressure in between).
+template <bool FUSED>
 __global__ void commit_kernel(ElemParams ep, double *y, const double *yout, double *P, double *Pdot,
                               const double *Ptemp, const double *Pdot_s, double *slip, const double *slip_out,
-                              int commit_p)
+                              const double *kbuf, double *ytmp, int commit_p, int B, const double *src_tb,
+                              double t_cap, unsigned int *ticket)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= ep.Ntot) return;
-    const int i = ep.inst_of[e];
-    const StepCtl &c = ep.ctl[i];
-    if (!takes_part(ep.ctl, i, M_ACTIVE) || !c.accepted || c.status != 0) return;
-    const Inst &I = ep.inst[i];
-    const int64_t N = I.N, k = e - I.eoff;
-    double *yi = y + 3 * I.eoff;
-    const double *yo = yout + 3 * I.eoff;
-    int bad = 0;
+    if (e < ep.Ntot) {
+        const int i = ep.inst_of[e];
+        const StepCtl &c = ep.ctl[i];
+        if (takes_part(ep.ctl, i, M_ACTIVE) && c.status == 0) {
+            const Inst &I = ep.inst[i];
+            const int64_t N = I.N, k = e - I.eoff;
+            double *yi = y + 3 * I.eoff;
+            bool accept = c.accepted;
+            double h = c.h;
+            if (FUSED) {
+                const Decision d = decide(c);
+                accept = d.accept;
+                h = d.h;
+            }
+            if (accept) {
+                const double *yo = yout + 3 * I.eoff;
+                int bad = 0;
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-        const double v = yo[j * N + k];
-        yi[j * N + k] = v;
-        if (j == 2 && v > 0.0) bad |= 1;
-        if (!isfinite(v)) bad |= 2;
+                for (int j = 0; j < 3; j++) {
+                    const double v = yo[j * N + k];
+                    yi[j * N + k] = v;
+                    if (j == 2 && v > 0.0) bad |= 1;
+                    if (!isfinite(v)) bad |= 2;
+                }
+                if (bad) atomicOr(&ep.ctl[i].commit_bad, bad);
+                if (slip) slip[e] = slip_out[e];
+                if (commit_p && !(c.pfail_mask & (1 << 4))) {
+                    P[e] = Ptemp[6 * I.eoff + 4 * N + k];
+                    Pdot[e] = Pdot_s[6 * I.eoff + 4 * N + k];
+                }
+            } else {
+                const double *kb = kbuf + 18 * I.eoff;
+                double *yt = ytmp + 3 * I.eoff;
+#pragma unroll
+                for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(2, h, yi[j * N + k], kb, 3 * N, j * N + k);
+            }
+        }
     }
-    if (bad) atomicOr(&ep.ctl[i].commit_bad, bad);
-    if (slip) slip[e] = slip_out[e];
-    if (commit_p && !(c.pfail_mask & (1 << 4))) {
-        P[e] = Ptemp[6 * I.eoff + 4 * N + k];
-        Pdot[e] = Pdot_s[6 * I.eoff + 4 * N + k];
+    if (FUSED) {
+        __shared__ bool last;
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        for (int i = threadIdx.x; i < B; i += blockDim.x) {
+            if (!takes_part(ep.ctl, i, M_ACTIVE)) continue;
+            StepCtl &c = ep.ctl[i];
+            ctl_decide(c, decide(c));
+            ctl_finish(c, ep.inst[i], src_tb, t_cap);
+        }
+        if (threadIdx.x == 0) *ticket = 0;
     }
 }
 
-// End of one pass of solve() per instance (src/solver.f90:117-196): time,
-// t_try with the 1-day cap, the stop rules on the committed state
-// (check_errors, src/solver.f90:412-418; non-finite values too) and the
-// instance's next phase.
-__global__ void finish_kernel(StepCtl *ctl, int B, double t_cap)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B || !takes_part(ctl, i, M_ACTIVE)) return;
-    StepCtl &c = ctl[i];
-    if (c.status != 0) { c.phase = PH_DONE; return; }
-    if (!c.accepted) { c.phase = PH_RETRY; return; }
-    c.time = c.time + c.hdid;
-    double tn = c.hnext;
-    if (tn > t_cap) tn = t_cap;
-    c.t_try = tn;
-    c.steps_done += 1;
-    if (c.commit_bad) {
-        c.status = (c.commit_bad & 1) ? 3 : 4;
-        c.phase = PH_DONE;
-        return;
-    }
-    bool done = (c.steps_done >= c.target_steps) || (c.t_end > 0.0 && c.time >= c.t_end * (1.0 - 1e-14));
-    c.phase = done ? PH_DONE : PH_NEW;
-}
-
-// Arms every instance for `nsteps` more accepted steps (or until t_end).
-__global__ void arm_kernel(StepCtl *ctl, int B, long long nsteps, double t_end, int max_attempts)
+// Arms every instance for `nsteps` more accepted steps (or until t_end) and
+// starts its first one.
+__global__ void arm_kernel(StepCtl *ctl, const Inst *inst, int B, const double *src_tb, long long nsteps, double t_end,
+                           int max_attempts)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= B) return;
@@ -2401,6 +2470,10 @@ __global__ void arm_kernel(StepCtl *ctl, int B, long long nsteps, double t_end, 
     c.t_end = t_end;
     c.max_attempts = max_attempts;
     c.phase = (c.status == 0 && nsteps > 0 && !(t_end > 0.0 && c.time >= t_end)) ? PH_NEW : PH_DONE;
+    if (c.phase == PH_NEW) {
+        ctl_step_begin(c, inst[i], src_tb);
+        ctl_attempt_begin(c);
+    }
 }
 
 // K.V output for the operator entry point: sum the chunks and scale.
