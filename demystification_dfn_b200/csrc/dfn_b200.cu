@@ -238,6 +238,24 @@ static gemv_tma_fn pick_gemv_tma(int mode, int store)
     return gemv_tma_kernel<3, 2>;
 }
 
+// Launch that may start while the kernel before it on the stream drains
+// (programmatic dependent launch; the kernel calls pdl_wait).
+template <typename... P, typename... A>
+static cudaError_t launch_pdl(void (*fn)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
 static const size_t kTmaSmem = TMA_STAGES * GEMV_CHUNK_BYTES + 2 * TMA_STAGES * sizeof(uint64_t);
 
 // H-matrix K.V: low-rank products, leaf rows, fixed-order row gather.
@@ -363,9 +381,8 @@ static void tc_launch_bn(dfn_handle *h, const TcOut &o)
     const unsigned units = (unsigned)(h->tc_nmt * h->tc_split);
     if (h->tc_variant == 0) {
         const unsigned grid = std::min(units, (unsigned)h->sms);
-        tc_gemm_persistent_kernel<BN, tc_stages(BN)><<<grid, TC_PTHREADS, tc_smem_bytes(BN, tc_stages(BN)),
-                                                       h->stream>>>(h->tc_A, h->tc_A + na, h->tc_B, h->tc_B + nb, o,
-                                                                    h->err_flag);
+        launch_pdl(tc_gemm_persistent_kernel<BN, tc_stages(BN)>, grid, TC_PTHREADS, tc_smem_bytes(BN, tc_stages(BN)),
+                   h->stream, h->tc_A, h->tc_A + na, h->tc_B, h->tc_B + nb, o, h->err_flag);
         return;
     }
     const unsigned grid = units;
@@ -381,8 +398,8 @@ static int launch_tc(dfn_handle *h, const double *Vbase, int vmul)
 {
     const Inst &I = h->hinst[0];
     const int64_t nb = (int64_t)h->tc_bn * h->tc_kpad;
-    tc_pack_v_kernel<<<blocks_of(nb, 256), 256, 0, h->stream>>>(Vbase, vmul, I.N, h->B, h->tc_bn, h->tc_kpad,
-                                                                h->tc_B, h->tc_B + nb);
+    CK(launch_pdl(tc_pack_v_kernel, blocks_of(nb, 256), 256, 0, h->stream, Vbase, vmul, I.N, h->B, h->tc_bn,
+                  h->tc_kpad, h->tc_B, h->tc_B + nb));
     h->launches++;
     CKL();
     TcOut o;
@@ -415,13 +432,14 @@ static int launch_s64(dfn_handle *h, int mask, const double *Vbase, int vmul)
 {
     const Inst &I = h->hinst[0];
     const S64Plan &pl = h->s64_pl;
-    s64_pack_v_kernel<<<dim3(blocks_of(I.Np, 256), (unsigned)(8 * pl.nt * pl.mtiles)), 256, 0, h->stream>>>(
-        Vbase, vmul, h->inst, I.N, h->B, I.Np, h->s64_vt);
+    CK(launch_pdl(s64_pack_v_kernel, dim3(blocks_of(I.Np, 256), (unsigned)(8 * pl.nt * pl.mtiles)), 256, 0, h->stream,
+                  Vbase, vmul, h->inst, I.N, h->B, I.Np, h->s64_vt));
     h->launches++;
     CKL();
     const s64_fn fn = h->mode == DFN_MODE_II ? pick_s64<2>(pl.nt) : pick_s64<3>(pl.nt);
-    fn<<<(unsigned)pl.ctas, S64_THREADS, s64_smem_bytes(h->mode, pl.nt), h->stream>>>(
-        static_cast<const double *>(h->K), h->s64_vt, h->inst, h->ctl, mask, I.N, I.Np, h->B, pl, h->partT, h->partN);
+    CK(launch_pdl(fn, (unsigned)pl.ctas, S64_THREADS, s64_smem_bytes(h->mode, pl.nt), h->stream,
+                  static_cast<const double *>(h->K), h->s64_vt, h->inst, h->ctl, mask, I.N, I.Np, h->B, pl, h->partT,
+                  h->partN));
     return DFN_OK;
 }
 
@@ -441,8 +459,8 @@ static int launch_gemv(dfn_handle *h, int mask, const double *Vbase, int vmul, b
         TRY(launch_s64(h, mask, Vbase, vmul));
     } else if (h->gemv_impl == 0) {
         gemv_tma_fn fn = pick_gemv_tma(h->mode, h->store);
-        fn<<<(unsigned)ntiles, (TMA_CONSUMERS + 1) * 32, kTmaSmem, h->stream>>>(
-            h->tiles, h->inst, h->ctl, mask, K, Vbase, vmul, h->partT, h->partN, h->wait_polls, h->err_flag);
+        CK(launch_pdl(fn, (unsigned)ntiles, (TMA_CONSUMERS + 1) * 32, kTmaSmem, h->stream, h->tiles, h->inst, h->ctl,
+                      mask, K, Vbase, vmul, h->partT, h->partN, h->wait_polls, h->err_flag));
     } else {
         gemv_fn fn = pick_gemv(h->mode, h->store);
         fn<<<(unsigned)ntiles, GEMV_WARPS * 32, 0, h->stream>>>(h->tiles, h->inst, h->ctl, mask, K, Vbase, vmul,
@@ -543,6 +561,8 @@ static int launch_pressure(dfn_handle *h, int mask, int kind, int sys0, int nsys
 static FricParams fric_params(dfn_handle *h, int64_t nelem)
 {
     FricParams f;
+    f.single = h->B == 1;
+    f.inst0 = h->hinst[0];
     f.Ntot = nelem; f.mode = h->mode; f.inst = h->inst; f.inst_of = h->inst_of;
     f.a = h->a; f.b = h->b; f.Dc = h->Dc; f.f0 = h->f0; f.V0 = h->V0; f.nload = h->nload; f.sload = h->sload;
     f.fake = h->fake; f.partT = h->partT; f.partN = h->partN; f.SigT = h->SigT; f.SigN = h->SigN;
@@ -555,15 +575,19 @@ static FricParams fric_params(dfn_handle *h, int64_t nelem)
     return f;
 }
 
-static int launch_friction(dfn_handle *h, int stage, int sys, int mask, int64_t nelem, double off_explicit = 0.0)
+// pdl = false: the stream has just waited for another one (the kernel would
+// read that one's results before its own wait).
+static int launch_friction(dfn_handle *h, int stage, int sys, int mask, int64_t nelem, double off_explicit = 0.0,
+                           bool pdl = true)
 {
     FricParams f = fric_params(h, nelem);
     f.off_explicit = off_explicit;
-    // 128-thread blocks: five per SM at the register count (two of 256)
-    if (h->form == DFN_FORM_NEWTON && h->guess == DFN_GUESS_MLP)
-        friction_kernel<true><<<(unsigned)((nelem + 127) / 128), 128, 0, h->stream>>>(f, stage, sys, mask);
-    else
-        friction_kernel<false><<<(unsigned)((nelem + 127) / 128), 128, 0, h->stream>>>(f, stage, sys, mask);
+    const unsigned grid = blocks_of(nelem, 128);
+    const bool fast = grid <= 3 * (unsigned)h->sms;   // one wave of the low-latency variant
+    auto fn = h->form == DFN_FORM_NEWTON && h->guess == DFN_GUESS_MLP ? friction_kernel<true, false>
+              : fast ? friction_kernel<false, true> : friction_kernel<false, false>;
+    if (pdl) CK(launch_pdl(fn, grid, 128, 0, h->stream, f, stage, sys, mask));
+    else fn<<<grid, 128, 0, h->stream>>>(f, stage, sys, mask);
     h->launches++;
     CKL();
     return DFN_OK;
@@ -627,7 +651,7 @@ static int run_stages(dfn_handle *h, int mask)
         TRY(launch_gemv(h, mask, h->ytmp, 3, false));
         if (s == 2 && after) TRY(launch_pressure_side(h, side, mask, 1, sys0, nsys, h->B));
         if (s == 2 && beside) CK(cudaStreamWaitEvent(h->stream, h->ev_pjoin, 0));
-        TRY(launch_friction(h, s, s - 1, mask, h->Ntot));
+        TRY(launch_friction(h, s, s - 1, mask, h->Ntot, 0.0, !(s == 2 && beside)));
     }
     return DFN_OK;
 }
@@ -687,13 +711,14 @@ static int run_round(dfn_handle *h)
     TRY(launch_gemv(h, M_NEW, h->Y, 3, false));
     if (after) TRY(launch_pressure_side(h, side, M_NEW, 0, 0, 1, h->B));
     if (beside) CK(cudaStreamWaitEvent(h->stream, h->ev_pjoin, 0));
-    TRY(launch_friction(h, 1, 0, M_NEW, h->Ntot));
+    TRY(launch_friction(h, 1, 0, M_NEW, h->Ntot, 0.0, !beside));
     TRY(run_stages(h, M_ACTIVE));
     if (h->pcoup) TRY(run_decide(h, M_ACTIVE));
-    (h->pcoup ? commit_kernel<false> : commit_kernel<true>)<<<blocks_of(h->Ntot, 256), 256, 0, h->stream>>>(
-        elem_params(h), h->Y, h->yout, h->P, h->Pdot, h->Ptemp, h->Pdot_s,
-        h->form == DFN_FORM_NEWTON ? nullptr : h->slip, h->slip_out, h->kbuf, h->ytmp, h->pcoup ? 0 : 1, h->B,
-        h->src_tb, h->max_step, h->ticket);
+    CK(launch_pdl(h->pcoup ? commit_kernel<false> : commit_kernel<true>,
+                  std::min(blocks_of(h->Ntot, 256), 8 * (unsigned)h->sms), 256, 0, h->stream,
+                  elem_params(h), h->Y, h->yout, h->P, h->Pdot, h->Ptemp, h->Pdot_s,
+                  h->form == DFN_FORM_NEWTON ? nullptr : h->slip, h->slip_out, h->kbuf, h->ytmp, h->pcoup ? 0 : 1,
+                  h->B, h->src_tb, h->max_step, h->ticket));
     h->launches++;
     CKL();
     if (h->pcoup) {

@@ -89,6 +89,17 @@ struct StepCtl {
 __device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
 
+// Programmatic dependent launch. A kernel launched with the attribute may
+// start while the kernel before it on the stream still runs; pdl_wait()
+// returns once that kernel has completed and its writes are visible, and
+// pdl_trigger() lets the next kernel start. Every kernel calls wait, then
+// trigger, in every block before it returns: when a kernel's wait returns,
+// all kernels before the previous one have completed too, so what comes
+// before the wait may read anything but the previous kernel's results.
+// Without the attribute the wait returns at once.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Stage abscissae: offset of stage s (1-based, s=2..6) from the step start.
 __device__ __forceinline__ double ck_a(int s)
 {
@@ -486,7 +497,17 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     __shared__ int issued_s, bad_s;
 
     const int4 t = tiles[blockIdx.x];
-    if (!takes_part(ctl, t.x, mask)) return;   // CTA-uniform: before any barrier
+    // a launch for networks at the start of a step follows the kernel that
+    // moves the controllers on, so its phases are read after the wait; the
+    // phases of a stage launch stand, and its copies of K (constant) start
+    // before the wait, beside the stage kernel that makes V
+    const bool early = mask != M_NEW;
+    if (!early) pdl_wait();
+    if (!takes_part(ctl, t.x, mask)) {   // CTA-uniform: before any barrier
+        if (early) pdl_wait();
+        pdl_trigger();
+        return;
+    }
     const Inst I = inst[t.x];
     const int64_t N = I.N;
     const unsigned char *K = reinterpret_cast<const unsigned char *>(Kbase + I.kvec);
@@ -506,7 +527,8 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     }
     __syncthreads();
     if (warp == TMA_CONSUMERS) {
-        // producer: one elected lane issues the bulk copies
+        // producer: one elected lane issues the bulk copies (it reads nothing
+        // that a kernel writes, so it does not wait for the previous one)
         if (lane == 0) {
             int i = 0;
             for (; i < nrows; i++) {
@@ -522,6 +544,8 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
             issued_s = i;
         }
     } else {
+        if (early) pdl_wait();
+        pdl_trigger();
         double v[GEMV_LPL * CPV];
 #pragma unroll
         for (int i = 0; i < GEMV_LPL; i++)
@@ -1816,6 +1840,8 @@ __global__ void __launch_bounds__(TRI_NT2, 1) pressure_tridiag_long_kernel(Press
 // Friction right-hand side fused with the Cash-Karp stage arithmetic.
 struct FricParams {
     int64_t Ntot;                 // elements of all instances
+    int single;                   // one instance: inst0, no table look-ups
+    Inst inst0;
     int mode;
     const Inst *inst;
     const int *inst_of;           // instance of each global element
@@ -1952,29 +1978,95 @@ __device__ __forceinline__ void newton_post(const FricParams &f, int64_t e, doub
     dpsi = V0 / Dc * exp(-psi) - fabs(V) / Dc;     // aging law, as the reference
 }
 
-__device__ __forceinline__ void rsf_rhs(const FricParams &f, int mode, int64_t e, double mu_2cs, double V, double psi,
-                                        double sig, double T, double Nn, double Pt, double Pd, double &dV,
-                                        double &dpsi, double &dsig)
+// Friction law with the state evolution, in two halves: what the slip rate,
+// log-state, pressure and normal traction give by themselves, then what needs
+// the stress rates (src/friction/RateStateAgingModeII.f90:46-76; mode III:
+// dsig = loading only). Operations are written out (no contraction left to
+// the compiler), so that every instantiation of the stage kernel rounds alike.
+struct RsfPre {
+    double as;       // a asinh(B C)
+    double w;        // B D (sig + P) b heal
+    double den, heal;
+};
+__device__ __forceinline__ RsfPre rsf_pre(double a, double b, double Dc, double f0, double V0, double mu_2cs, double V,
+                                          double psi, double sig, double Pt)
 {
-    // src/friction/RateStateAgingModeII.f90:46-76 (mode III: dsig = loading only)
-    dsig = (mode == 2) ? (Nn + f.nload[e]) : f.nload[e];
-    const double a = f.a[e], b = f.b[e], V0 = f.V0[e], Dc = f.Dc[e];
-    double B = V / (2.0 * V0);
-    double C = exp((f.f0[e] + b * psi) / a);
-    double D = 1.0 / (C * C) + B * B;
-    D = 1.0 / sqrt(D);
-    double heal = V0 / Dc * exp(-psi) - fabs(V) / Dc;
-    double num = f.sload[e] + T + (dsig + Pd) * a * asinh(B * C) + B * D * (sig + Pt) * b * heal;
-    double den = mu_2cs - D * (sig + Pt) * a / (2.0 * V0);
-    dV = num / den;
-    dpsi = heal;
-    if (f.fake[e]) { dV = 0.0; dpsi = 0.0; dsig = 0.0; }
+    RsfPre r;
+    const double v2 = 2.0 * V0;
+    const double B = __ddiv_rn(V, v2);
+    const double x = __ddiv_rn(__fma_rn(b, psi, f0), a);
+    const double C = exp(x);
+    const double D = rsqrt(__fma_rn(B, B, __ddiv_rn(1.0, mul_(C, C))));
+    const double z = mul_(B, C), az = fabs(z);
+    // asinh z = sign(z) ln(2|z|) to 1/(4 z^2): with z = B e^x no exponential
+    // has to be taken back by a logarithm (the usual case: a asinh z is the
+    // friction coefficient, z ~ e^60)
+    double ash;
+    if (az > 1.0e9 && az < 1.0e300) ash = copysign(add_(add_(log(fabs(B)), x), 0.6931471805599453), z);
+    else if (az == 0.0) ash = z;   // fake elements: most warps hold one
+    else ash = asinh(z);
+    r.as = mul_(a, ash);
+    r.heal = __ddiv_rn(__fma_rn(V0, exp(-psi), -fabs(V)), Dc);
+    const double s = add_(sig, Pt), Ds = mul_(D, s);
+    r.w = mul_(mul_(mul_(B, Ds), b), r.heal);
+    r.den = add_(mu_2cs, -__ddiv_rn(mul_(Ds, a), v2));
+    return r;
+}
+__device__ __forceinline__ double rsf_dV(const RsfPre &r, double sload, double T, double dsig, double Pd)
+{
+    return __ddiv_rn(add_(__fma_rn(add_(dsig, Pd), r.as, add_(sload, T)), r.w), r.den);
 }
 
 __device__ __forceinline__ void atomic_max_pos(unsigned long long *addr, double v)
 {
     // non-negative doubles order like their bit patterns
     atomicMax(addr, (unsigned long long)__double_as_longlong(v));
+}
+
+// Sum of the column-chunk partials of an element, in chunk order; eight
+// loads in flight (they would otherwise wait for one another's additions).
+__device__ __forceinline__ double sum_chunks(const double *p, int n, int64_t stride)
+{
+    double s = 0.0;
+    for (; n >= 8; n -= 8) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) { v[q] = *p; p += stride; }
+#pragma unroll
+        for (int q = 0; q < 8; q++) s += v[q];
+    }
+    for (; n >= 2; n -= 2) {
+        const double v0 = p[0], v1 = p[stride];
+        s += v0;
+        s += v1;
+        p += 2 * stride;
+    }
+    if (n) s += *p;
+    return s;
+}
+
+// Cash-Karp sum over k1 .. k_{n} of one component for the ytemp of stage
+// n + 2, without its last term k_{n+1} (n = stage - 1 terms; the reference's
+// operand order, src/ode_solver/ode_bs.f90:213-221).
+__device__ __forceinline__ double ck_head(int n, const double *k)
+{
+    switch (n) {
+    case 0: return 0.0;
+    case 1: return mul_(CK_B31, k[0]);
+    case 2: return add_(mul_(CK_B41, k[0]), mul_(CK_B42, k[1]));
+    case 3: return add_(add_(mul_(CK_B51, k[0]), mul_(CK_B52, k[1])), mul_(CK_B53, k[2]));
+    default:
+        return add_(add_(add_(mul_(CK_B61, k[0]), mul_(CK_B62, k[1])), mul_(CK_B63, k[2])), mul_(CK_B64, k[3]));
+    }
+}
+__device__ __forceinline__ double ck_last(int n)
+{
+    switch (n) {
+    case 1: return CK_B32;
+    case 2: return CK_B43;
+    case 3: return CK_B54;
+    default: return CK_B65;
+    }
 }
 
 // stage: 0 = standalone evaluation (ytmp in, kbuf slot 0 out)
@@ -1985,48 +2077,48 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long *addr, double 
 // LEARNED: Newton formulation with the learned guess (a separate
 // instantiation keeps the tensor-core inference's registers out of the
 // other variants).
-// Without the learned guess the kernel is held to 64 registers (8 blocks of
-// 128 threads per SM, 136 bytes of spills to L1): it waits on memory, and
-// the extra warps raise the tensor-core round by 5-6 % over 5 blocks at 84
-// registers.
-template <bool LEARNED>
-__global__ void __launch_bounds__(128, LEARNED ? 5 : 8) friction_kernel(FricParams f, int stage, int sys, int mask)
+// FAST: launches that fit in one wave at three blocks per SM, where the
+// kernel is a chain of latencies: all loads but the K.V partials, the
+// friction law's transcendentals and the Cash-Karp sums of the earlier stages
+// come before the wait for the K.V kernel, beside which they run (4-fault
+// network, 20 steps: 3.38 -> 2.57 ms with the K.V kernel's copies of K before
+// its wait; 4000-element fault, 16 steps: 3.84 -> 3.15 ms).
+// Otherwise the kernel is held to 64 registers (8 blocks of 128 threads per
+// SM) and loads where it needs: it waits on memory, and the extra warps raise
+// the tensor-core round by 5-6 % over 5 blocks at 84 registers. Its 64 members
+// of 16 013 elements are bound by issue (FP64 functions and divisions):
+// 1173 -> 1093 instructions per element and 86 -> 76 us in stage 2.
+template <bool LEARNED, bool FAST>
+__global__ void __launch_bounds__(128, LEARNED ? 5 : (FAST ? 3 : 8)) friction_kernel(FricParams f, int stage, int sys,
+                                                                                     int mask)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     int myi = -1;
     int nit = 0, nsolve = 0, nfail = 0;
     double emax = 0.0;
     if (e < f.Ntot) {
-        const int i = f.inst_of[e];
+        const int i = f.single ? 0 : f.inst_of[e];
         if (takes_part(f.ctl, i, mask)) myi = i;
     }
-    // phase 1: stresses, stage state and pressure; for the Newton
-    // formulation the analytic start and the network inputs
-    double T = 0.0, Nn = 0.0, V = 0.0, psi = 0.0, sig = 0.0, Pt = 0.0, Pd = 0.0;
-    NPre q;
-    q.kind = 0;
-    q.need = false;
-    q.big = false;
-#pragma unroll
-    for (int i = 0; i < MLP_IN; i++) q.x[i] = 0.0f;
-    if (myi >= 0) {
-        const Inst &I = f.inst[myi];
-        const int64_t N = I.N, k = e - I.eoff;
-        const StepCtl *ctl = f.ctl + myi;
-        const double *pT = f.partT + I.poff + k;
-        for (int64_t c = 0; c < I.nchunk; c++) T += pT[c * N];
-        T = I.prefT * T;
-        if (f.mode == 2) {
-            const double *pN = f.partN + I.poff + k;
-            for (int64_t c = 0; c < I.nchunk; c++) Nn += pN[c * N];
-            Nn = I.prefT * Nn;
-        }
-        f.SigT[e] = T;
-        f.SigN[e] = Nn;
-        const double *yin = (stage == 1) ? f.y + 3 * I.eoff : f.ytmp + 3 * I.eoff;
+    const bool on = myi >= 0;
+    const Inst &I = f.single ? f.inst0 : f.inst[on ? myi : 0];
+    const int64_t N = I.N, eoff = I.eoff, k = e - eoff, S = 3 * N;
+    const double mu_2cs = I.mu_2cs;
+    StepCtl *ctl = f.ctl + (on ? myi : 0);
+    // phase 1: stage state, pressure and what follows from them
+    double V = 0.0, psi = 0.0, sig = 0.0, Pt = 0.0, Pd = 0.0, hh = 0.0, tt = 0.0;
+    double y0[3] = {0.0, 0.0, 0.0}, head[3], ehead[3];
+    double p_nload = 0.0, p_sload = 0.0;
+    bool fake = false;
+    RsfPre rp{};
+    const double *yi = f.y + 3 * eoff;
+    double *yt = f.ytmp + 3 * eoff;
+    double *kb = f.kbuf + 18 * eoff;
+    auto load_state = [&]() {
+        const double *yin = (stage == 1) ? yi : yt;
         V = yin[k]; psi = yin[N + k]; sig = yin[2 * N + k];
-        Pt = f.Ptemp[6 * I.eoff + (int64_t)sys * N + k];
-        Pd = f.Pdot[6 * I.eoff + (int64_t)sys * N + k];
+        Pt = f.Ptemp[6 * eoff + (int64_t)sys * N + k];
+        Pd = f.Pdot[6 * eoff + (int64_t)sys * N + k];
         if (f.form == 1 && stage >= 1) {
             // Newton formulation: the stress balance uses P itself, so the
             // stage pressure must be smooth in the stage time. It is linear
@@ -2034,15 +2126,69 @@ __global__ void __launch_bounds__(128, LEARNED ? 5 : 8) friction_kernel(FricPara
             // the whole step (system 4, c = 1), which is what is committed.
             // (stage 1 takes P itself: the full-step system of this attempt
             // is not solved yet)
-            const double p0 = f.Pc[I.eoff + k];
-            Pt = (stage == 1) ? p0 : add_(p0, mul_(ck_a(stage), f.Ptemp[6 * I.eoff + 4 * N + k] - p0));
+            const double p0 = f.Pc[eoff + k];
+            Pt = (stage == 1) ? p0 : add_(p0, mul_(ck_a(stage), f.Ptemp[6 * eoff + 4 * N + k] - p0));
         }
+        hh = (stage == 1) ? ctl->t_try : ctl->h;
         if (f.form == 1) {
             const double off = (stage == 0) ? f.off_explicit
                                             : (stage == 1 ? 0.0 : add_(ctl->x, mul_(ck_a(stage), ctl->h)));
-            const double tt = (ctl->time - I.t0) + off;
-            newton_pre(f, e, f.mode, I.mu_2cs, tt, psi, sig, T, Nn, Pt, q);
+            tt = (ctl->time - I.t0) + off;
         }
+        p_nload = f.nload[e];
+        p_sload = f.sload[e];
+        fake = f.fake[e];
+    };
+    auto pre_rsf = [&]() {
+        if (f.form == 0)
+            rp = rsf_pre(f.a[e], f.b[e], f.Dc[e], f.f0[e], f.V0[e], mu_2cs, V, psi, sig, Pt);
+    };
+    auto load_heads = [&]() {
+        if (stage == 0) return;
+        double kk[3][5];
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            y0[j] = yi[j * N + k];
+#pragma unroll
+            for (int q = 0; q < 5; q++) kk[j][q] = (q < stage - 1) ? kb[q * S + j * N + k] : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            if (stage < 6) {
+                head[j] = ck_head(stage - 1, kk[j]);
+            } else {
+                // src/ode_solver/ode_bs.f90:223-224
+                head[j] = add_(add_(mul_(CK_C1, kk[j][0]), mul_(CK_C3, kk[j][2])), mul_(CK_C4, kk[j][3]));
+                ehead[j] = add_(add_(add_(mul_(CK_DC1, kk[j][0]), mul_(CK_DC3, kk[j][2])), mul_(CK_DC4, kk[j][3])),
+                                mul_(CK_DC5, kk[j][4]));
+            }
+        }
+    };
+    if (FAST && on) {
+        load_state();
+        load_heads();
+        pre_rsf();
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (!__any_sync(0xffffffffu, on)) return;
+    if (!FAST && on) {
+        load_state();
+        pre_rsf();
+    }
+    double T = 0.0, Nn = 0.0;
+    NPre q;
+    q.kind = 0;
+    q.need = false;
+    q.big = false;
+#pragma unroll
+    for (int i = 0; i < MLP_IN; i++) q.x[i] = 0.0f;
+    if (on) {
+        T = I.prefT * sum_chunks(f.partT + I.poff + k, (int)I.nchunk, N);
+        if (f.mode == 2) Nn = I.prefT * sum_chunks(f.partN + I.poff + k, (int)I.nchunk, N);
+        f.SigT[e] = T;
+        f.SigN[e] = Nn;
+        if (f.form == 1) newton_pre(f, e, f.mode, mu_2cs, tt, psi, sig, T, Nn, Pt, q);
     }
     // the learned guess: evaluated only by warps that hold an element whose
     // analytic start misses the tolerance by more than the gate; the
@@ -2054,70 +2200,60 @@ __global__ void __launch_bounds__(128, LEARNED ? 5 : 8) friction_kernel(FricPara
         if (__any_sync(0xffffffffu, q.big)) {
             ym = mlp_warp_tc_call(f.mlp, q.x[0], q.x[1], q.x[2], q.x[3], q.x[4], q.x[5], q.x[6]);
             have_ym = true;
-            if ((threadIdx.x & 31) == 0 && myi >= 0) atomicAdd((unsigned long long *)&f.ctl[myi].mlp_warps, 1ull);
+            if ((threadIdx.x & 31) == 0 && on) atomicAdd((unsigned long long *)&f.ctl[myi].mlp_warps, 1ull);
         }
     }
     // phase 2: derivatives and the Cash-Karp stage arithmetic
-    if (myi >= 0) {
-        const Inst &I = f.inst[myi];
-        const int64_t N = I.N, k = e - I.eoff, S = 3 * N;
-        StepCtl *ctl = f.ctl + myi;
-        const double *yi = f.y + 3 * I.eoff;
-        double *yt = f.ytmp + 3 * I.eoff;
-        double dV, dpsi, dsig;
+    if (on) {
+        double d[3];   // dV (or dslip), dpsi, dsigma
         if (f.form == 1) {
             int ok = 1;
-            newton_post(f, e, I.mu_2cs, psi, q, ym, have_ym, dV, dpsi, dsig, nit, ok);
-            nsolve = f.fake[e] ? 0 : 1;
+            newton_post(f, e, mu_2cs, psi, q, ym, have_ym, d[0], d[1], d[2], nit, ok);
+            nsolve = fake ? 0 : 1;
             nfail = ok ? 0 : 1;
         } else {
-            rsf_rhs(f, f.mode, e, I.mu_2cs, V, psi, sig, T, Nn, Pt, Pd, dV, dpsi, dsig);
+            d[2] = (f.mode == 2) ? add_(Nn, p_nload) : p_nload;
+            d[0] = rsf_dV(rp, p_sload, T, d[2], Pd);
+            d[1] = rp.heal;
+            if (fake) { d[0] = 0.0; d[1] = 0.0; d[2] = 0.0; }
         }
-        double *kb = f.kbuf + 18 * I.eoff;
-        const int slot = (stage == 0) ? 0 : stage - 1;
-        double *ks = kb + (int64_t)slot * S;
-        ks[k] = dV; ks[N + k] = dpsi; ks[2 * N + k] = dsig;
+        if (!FAST) load_heads();
+        double *ks = kb + (int64_t)(stage == 0 ? 0 : stage - 1) * S;
+#pragma unroll
+        for (int j = 0; j < 3; j++) ks[j * N + k] = d[j];
         if (stage == 1) {
-            const double tt = ctl->t_try, tol = ctl->eps;
-            double *ysc = f.yscal + 3 * I.eoff;
-            // yscal = abs(Y)+abs(Y_dot*t_try)+tol_solver (src/solver.f90:102)
-            ysc[k] = add_(add_(fabs(yi[k]), fabs(mul_(dV, tt))), tol);
-            ysc[N + k] = add_(add_(fabs(yi[N + k]), fabs(mul_(dpsi, tt))), tol);
-            ysc[2 * N + k] = add_(add_(fabs(yi[2 * N + k]), fabs(mul_(dsig, tt))), tol);
+            const double tol = ctl->eps;
+            double *ysc = f.yscal + 3 * eoff;
+            // yscal = abs(Y)+abs(Y_dot*t_try)+tol_solver (src/solver.f90:102);
             // the first attempt's step is t_try: ytemp of stage 2
 #pragma unroll
-            for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(2, tt, yi[j * N + k], kb, S, j * N + k);
-            if (k == 0) ctl->h = tt;   // read by later launches only
+            for (int j = 0; j < 3; j++) {
+                ysc[j * N + k] = add_(add_(fabs(y0[j]), fabs(mul_(d[j], hh))), tol);
+                yt[j * N + k] = add_(y0[j], mul_(mul_(CK_B21, hh), d[j]));
+            }
+            if (k == 0) ctl->h = hh;   // read by later launches only
         } else if (stage >= 2 && stage <= 5) {
-            const double h = ctl->h;
 #pragma unroll
-            for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(stage + 1, h, yi[j * N + k], kb, S, j * N + k);
+            for (int j = 0; j < 3; j++)
+                yt[j * N + k] = add_(y0[j], mul_(hh, add_(head[j], mul_(ck_last(stage - 1), d[j]))));
         }
         if (f.form == 0 && stage >= 3) {
             // slip of the V formulation: k_s(slip) = V of the stage input,
             // 5th-order combination in the reference's operand order
             // (src/ode_solver/ode_bs.f90:223), outside the error norm
-            if (stage == 3) f.slip_acc[e] = add_(mul_(CK_C1, yi[k]), mul_(CK_C3, V));
+            if (stage == 3) f.slip_acc[e] = add_(mul_(CK_C1, y0[0]), mul_(CK_C3, V));
             else if (stage == 4) f.slip_acc[e] = add_(f.slip_acc[e], mul_(CK_C4, V));
             else if (stage == 6)
-                f.slip_out[e] = add_(f.slip[e], mul_(ctl->h, add_(f.slip_acc[e], mul_(CK_C6, V))));
+                f.slip_out[e] = add_(f.slip[e], mul_(hh, add_(f.slip_acc[e], mul_(CK_C6, V))));
         }
         if (stage == 6) {
-            const double h = ctl->h;
-            const double *ysc = f.yscal + 3 * I.eoff;
-            double *yo = f.yout + 3 * I.eoff;
+            const double *ysc = f.yscal + 3 * eoff;
+            double *yo = f.yout + 3 * eoff;
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                const int64_t q = j * N + k;
-                const double k1 = kb[q], k3 = kb[2 * S + q], k4 = kb[3 * S + q], k5 = kb[4 * S + q],
-                             k6 = kb[5 * S + q];
-                // src/ode_solver/ode_bs.f90:223-224
-                yo[q] = add_(yi[q], mul_(h, add_(add_(add_(mul_(CK_C1, k1), mul_(CK_C3, k3)), mul_(CK_C4, k4)),
-                                                 mul_(CK_C6, k6))));
-                double yerr = mul_(h, add_(add_(add_(add_(mul_(CK_DC1, k1), mul_(CK_DC3, k3)), mul_(CK_DC4, k4)),
-                                                mul_(CK_DC5, k5)),
-                                           mul_(CK_DC6, k6)));
-                double er = fabs(__ddiv_rn(yerr, ysc[q]));
+                yo[j * N + k] = add_(y0[j], mul_(hh, add_(head[j], mul_(CK_C6, d[j]))));
+                const double yerr = mul_(hh, add_(ehead[j], mul_(CK_DC6, d[j])));
+                double er = fabs(__ddiv_rn(yerr, ysc[j * N + k]));
                 if (!(er == er) || isinf(er)) er = 1.0e300;   // non-finite error rejects the attempt
                 emax = fmax(emax, er);
             }
@@ -2400,50 +2536,61 @@ __global__ void commit_kernel(ElemParams ep, double *y, const double *yout, doub
                               const double *kbuf, double *ytmp, int commit_p, int B, const double *src_tb,
                               double t_cap, unsigned int *ticket)
 {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e < ep.Ntot) {
+    pdl_wait();
+    pdl_trigger();
+    // blocks walk the elements: few of them for the fence at the end
+    int last_i = -1;
+    Decision d{};
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ep.Ntot;
+         e += (int64_t)gridDim.x * blockDim.x) {
         const int i = ep.inst_of[e];
         const StepCtl &c = ep.ctl[i];
         if (takes_part(ep.ctl, i, M_ACTIVE) && c.status == 0) {
             const Inst &I = ep.inst[i];
             const int64_t N = I.N, k = e - I.eoff;
             double *yi = y + 3 * I.eoff;
-            bool accept = c.accepted;
-            double h = c.h;
-            if (FUSED) {
-                const Decision d = decide(c);
-                accept = d.accept;
-                h = d.h;
+            if (i != last_i) {
+                if (FUSED) {
+                    d = decide(c);
+                } else {
+                    d.accept = c.accepted;
+                    d.h = c.h;
+                }
+                last_i = i;
             }
-            if (accept) {
+            if (d.accept) {
+                // all loads before the stores, which might alias them
                 const double *yo = yout + 3 * I.eoff;
-                int bad = 0;
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    const double v = yo[j * N + k];
-                    yi[j * N + k] = v;
-                    if (j == 2 && v > 0.0) bad |= 1;
-                    if (!isfinite(v)) bad |= 2;
+                const bool cp = commit_p && !(c.pfail_mask & (1 << 4));
+                const double v0 = yo[k], v1 = yo[N + k], v2 = yo[2 * N + k];
+                const double sl = slip ? slip_out[e] : 0.0;
+                const double pt = cp ? Ptemp[6 * I.eoff + 4 * N + k] : 0.0;
+                const double pd = cp ? Pdot_s[6 * I.eoff + 4 * N + k] : 0.0;
+                yi[k] = v0;
+                yi[N + k] = v1;
+                yi[2 * N + k] = v2;
+                if (slip) slip[e] = sl;
+                if (cp) {
+                    P[e] = pt;
+                    Pdot[e] = pd;
                 }
+                const int bad = (v2 > 0.0 ? 1 : 0) | (isfinite(v0) && isfinite(v1) && isfinite(v2) ? 0 : 2);
                 if (bad) atomicOr(&ep.ctl[i].commit_bad, bad);
-                if (slip) slip[e] = slip_out[e];
-                if (commit_p && !(c.pfail_mask & (1 << 4))) {
-                    P[e] = Ptemp[6 * I.eoff + 4 * N + k];
-                    Pdot[e] = Pdot_s[6 * I.eoff + 4 * N + k];
-                }
             } else {
                 const double *kb = kbuf + 18 * I.eoff;
                 double *yt = ytmp + 3 * I.eoff;
 #pragma unroll
-                for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(2, h, yi[j * N + k], kb, 3 * N, j * N + k);
+                for (int j = 0; j < 3; j++) yt[j * N + k] = ck_combine(2, d.h, yi[j * N + k], kb, 3 * N, j * N + k);
             }
         }
     }
     if (FUSED) {
         __shared__ bool last;
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        __syncthreads();   // the block has read the controllers and raised its flags
+        if (threadIdx.x == 0) {
+            __threadfence();
+            last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        }
         __syncthreads();
         if (!last) return;
         __threadfence();

@@ -47,7 +47,10 @@ constexpr int S64_ROWS = 64;
 constexpr int S64_COLS = 16;
 constexpr int S64_THREADS = 128;
 constexpr int S64_NT = 8;                        // at most 8 tiles of 8 members per CTA
-constexpr int S64_MIN_STEPS = 8;                 // chunks a CTA gets at least
+// Chunks a CTA gets at least. A chunk takes about 0.8 us, so small matrices
+// are spread thin: N = 305, R = 43 takes 31 / 16.5 / 14.5 / 14.4 us with 8 / 4
+// / 2 / 1 (one only adds partial sums); from N = 2000 on no difference.
+constexpr int S64_MIN_STEPS = 2;
 constexpr int S64_VROW = S64_COLS + 4;           // doubles of a staged V row (160 bytes)
 
 // doubles of a staged K row: 320 bytes (mode II) or 160
@@ -140,6 +143,8 @@ __global__ void s64_pack_v_kernel(const double *__restrict__ Vbase, int vmul, co
 {
     const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int m = blockIdx.y;
+    pdl_wait();
+    pdl_trigger();
     if (l >= Np) return;
     vt[(int64_t)m * Np + l] = (l < N && m < R) ? Vbase[(int64_t)vmul * inst[m].eoff + l] : 0.0;
 }
@@ -157,6 +162,8 @@ __global__ void __launch_bounds__(S64_THREADS, 2)
     constexpr int ST = s64_stages(MODE, NT);
     extern __shared__ __align__(16) double s64_smem[];
 
+    pdl_wait();
+    pdl_trigger();
     if (!any_takes_part(ctl, R, mask)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;

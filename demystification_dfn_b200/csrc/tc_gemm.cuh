@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(TC_PTHREADS, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();   // the packed V; the set-up above runs beside its kernel
 
     if (warp == 0) {
         if (lane == 0) {
@@ -421,6 +422,8 @@ __global__ void tc_pack_v_kernel(const double *__restrict__ Vbase, int vmul, int
                                  int64_t kpad, __nv_bfloat16 *__restrict__ Bh, __nv_bfloat16 *__restrict__ Bl)
 {
     const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     if (idx >= (int64_t)rpad * kpad) return;
     const int r = (int)(idx / kpad);
     const int64_t l = idx - (int64_t)r * kpad;
