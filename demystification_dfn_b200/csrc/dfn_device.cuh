@@ -96,7 +96,9 @@ __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a,
 // trigger, in every block before it returns: when a kernel's wait returns,
 // all kernels before the previous one have completed too, so what comes
 // before the wait may read anything but the previous kernel's results.
-// Without the attribute the wait returns at once.
+// Without the attribute the wait returns at once. What an earlier kernel of
+// the chain writes is no __restrict__ const parameter here: such loads count
+// as invariant and may be moved before the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -483,8 +485,8 @@ __device__ __forceinline__ void tma_bulk_g2s(void *dst, const void *src, uint32_
 // round-robin, one stage per row (stage s is always read by warp s % 8).
 template <int MODE, int STORE>
 __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
-    gemv_tma_kernel(const int4 *__restrict__ tiles, const Inst *__restrict__ inst, const StepCtl *__restrict__ ctl,
-                    int mask, const uint4 *__restrict__ Kbase, const double *__restrict__ Vbase, int vmul,
+    gemv_tma_kernel(const int4 *__restrict__ tiles, const Inst *__restrict__ inst, const StepCtl *ctl,
+                    int mask, const uint4 *__restrict__ Kbase, const double *Vbase, int vmul,
                     double *__restrict__ partT, double *__restrict__ partN, int wait_polls, int *err_flag)
 {
     constexpr int BPC = KFmt<MODE, STORE>::BPC;

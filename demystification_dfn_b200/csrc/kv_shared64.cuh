@@ -138,7 +138,7 @@ __device__ __forceinline__ bool any_takes_part(const StepCtl *ctl, int R, int ma
 
 // vt[m * Np + l] = V of member m at column l (zero beyond N and R); V of
 // member m is Vbase[vmul * eoff_m + l]. grid (ceil(Np / 256), RP)
-__global__ void s64_pack_v_kernel(const double *__restrict__ Vbase, int vmul, const Inst *__restrict__ inst,
+__global__ void s64_pack_v_kernel(const double *Vbase, int vmul, const Inst *__restrict__ inst,
                                   int64_t N, int R, int64_t Np, double *__restrict__ vt)
 {
     const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -151,8 +151,8 @@ __global__ void s64_pack_v_kernel(const double *__restrict__ Vbase, int vmul, co
 
 template <int MODE, int NT>
 __global__ void __launch_bounds__(S64_THREADS, 2)
-    s64_gemm_kernel(const double *__restrict__ K, const double *__restrict__ vt, const Inst *__restrict__ inst,
-                    const StepCtl *__restrict__ ctl, int mask, int64_t N, int64_t Np, int R, S64Plan pl,
+    s64_gemm_kernel(const double *__restrict__ K, const double *vt, const Inst *__restrict__ inst,
+                    const StepCtl *ctl, int mask, int64_t N, int64_t Np, int R, S64Plan pl,
                     double *__restrict__ partT, double *__restrict__ partN)
 {
     constexpr int CPE = (MODE == 2) ? 2 : 1;             // doubles per stored entry

@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(TC_PTHREADS, 1)
     tc_gemm_persistent_kernel(const __nv_bfloat16 *__restrict__ Ah, const __nv_bfloat16 *__restrict__ Al,
-                              const __nv_bfloat16 *__restrict__ Bh, const __nv_bfloat16 *__restrict__ Bl, TcOut out,
+                              const __nv_bfloat16 *Bh, const __nv_bfloat16 *Bl, TcOut out,
                               int *err_flag)
 {
     static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "N of an M=128 MMA is a multiple of 16 up to 256");
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(TC_PTHREADS, 1)
 // V of the R networks of a stage -> BF16 hi/lo, swizzled tiles of rpad rows
 // per 64 reduction elements (zero padded); V of network r is
 // Vbase[vmul * r * N + l]. One thread per (row, element).
-__global__ void tc_pack_v_kernel(const double *__restrict__ Vbase, int vmul, int64_t N, int R, int rpad,
+__global__ void tc_pack_v_kernel(const double *Vbase, int vmul, int64_t N, int R, int rpad,
                                  int64_t kpad, __nv_bfloat16 *__restrict__ Bh, __nv_bfloat16 *__restrict__ Bl)
 {
     const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
