@@ -93,7 +93,7 @@ struct dfn_handle {
     bool use_graphs = true;
     int B = 1;                    // networks in the batch
     int mode = 2, store = 0, pressure = 0, gemv_impl = 0, max_attempts = 64;
-    int64_t Ntot = 0;             // elements of all networks
+    int64_t Ntot = 0, nmax = 0;   // elements of all networks, of the largest
     std::vector<Inst> hinst;      // host copy of the instance table
     Inst *inst = nullptr;
     int *inst_of = nullptr;
@@ -492,6 +492,13 @@ static void pcl_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int cl,
     cfg.numAttrs = 1;
 }
 
+// The one-CTA CG with its vectors in registers: the same results as on global
+// memory for networks of at most two elements per thread.
+static bool cg_small(const dfn_handle *h)
+{
+    return h->pressure == DFN_PRESSURE_CG && h->ncross == 0 && h->nmax <= 2 * CGS_THREADS;
+}
+
 static int launch_pressure(dfn_handle *h, int mask, int kind, int sys0, int nsys, double dt_explicit, int ninst)
 {
     const bool clusters = h->pcl > 0 && (h->pcl_mode == 1 || (h->pcl_mode < 0 && nsys * ninst <= h->pcl_max));
@@ -503,6 +510,11 @@ static int launch_pressure(dfn_handle *h, int mask, int kind, int sys0, int nsys
         pcl_config(cfg, at, cl, h->pcl_n, h->pcl_lean, (unsigned)(nsys * cl), (unsigned)ninst, h->stream);
         CK(cudaLaunchKernelEx(&cfg, pressure_cg_cluster_kernel, h->pg, (const Inst *)h->inst, h->ctl, mask, kind,
                               sys0, dt_explicit, h->Ptemp, h->Pdot_s, h->pwork, h->pcl_lean ? 1 : 0, h->pcoef));
+    } else if (cg_small(h)) {
+        dim3 grid((unsigned)nsys, (unsigned)ninst);
+        const unsigned nt = 32 * blocks_of(std::min<int64_t>(h->nmax, CGS_THREADS), 32);
+        (h->nmax <= CGS_THREADS ? pressure_cg_small_kernel<1> : pressure_cg_small_kernel<2>)<<<grid, nt, 0, h->stream>>>(
+            h->pg, h->inst, h->ctl, mask, kind, sys0, dt_explicit, h->Ptemp, h->Pdot_s, h->pwork);
     } else if (h->pressure != DFN_PRESSURE_TRIDIAG) {
         dim3 grid((unsigned)nsys, (unsigned)ninst);
         const int exact = h->pressure == DFN_PRESSURE_CG_EXACT ? 1 : 0;
@@ -604,8 +616,8 @@ static ElemParams elem_params(dfn_handle *h)
 // Pressure solves beside the K.V that follows them (they depend only on the
 // stage times, not on the stage state); the stage kernel that reads them
 // waits for the join. Returns the stream: the high-priority one for the CG on
-// a few thread-block clusters (at most half the SMs: placed first, the K.V
-// streams on the others), the lowest-priority one for the tiled tridiagonal
+// a few thread-block clusters or CTAs (at most half the SMs: placed first, the
+// K.V streams on the others) and for a few long tridiagonal segments, the lowest-priority one for the tiled tridiagonal
 // solve of a tensor-core batch (one tile CTA fits beside each persistent GEMM
 // CTA; issued after the GEMM, so that the GEMM's CTAs are placed first and the
 // tiles fill around them), or none (in line). The fork event is recorded
@@ -618,6 +630,8 @@ static cudaStream_t pressure_beside(dfn_handle *h, int nsys, int ninst)
         // long segments alone, a CTA each
         return (h->nshort == 0 && nsys * h->nlong <= h->sms / 2) ? h->side_stream : nullptr;
     }
+    if (cg_small(h) && h->pcl_mode <= 0 && h->pcl == 0)
+        return (int64_t)nsys * ninst <= h->sms / 2 ? h->side_stream : nullptr;   // a CTA each
     if (h->pressure != DFN_PRESSURE_CG || h->pcl <= 0 || h->pcl_mode == 0 || h->pcl_mode == 2) return nullptr;
     if (h->pcl_mode < 0 && (int64_t)nsys * ninst > h->pcl_max) return nullptr;
     return ((int64_t)nsys * ninst * h->pcl <= h->sms / 2) ? h->side_stream : nullptr;
@@ -1620,6 +1634,7 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
         I.tol = p.tol_solver;
         I.t0 = p.time0;
         eoff += I.N;
+        h->nmax = std::max(h->nmax, I.N);
         if (!h->hmat && !h->tc && !h->s64) kvec += I.N * I.Np * bpc / 16;
         if (h->s64 && i == 0) kvec = I.N * I.Np * bpc / 16;
         poff += I.nchunk * I.N;

@@ -1004,22 +1004,23 @@ __device__ int cg_solve(const PressParams &p, double dt, double *x, double *r, d
 }
 
 // One system of the reference CG for one instance (whole CTA), shared by
-// the batched solver and the allocation-free entry point.
-template <bool XC = false>
-__device__ void cg_system(const PressParams &p, StepCtl *ctl, int kind, int sys, double dt_explicit, double *Pt,
-                          double *Pd, double *x, double *r, double *pv, double *Mp, double *red, long long *iters,
-                          int exact, double *cf = nullptr)
+// the solvers: solve(dt) leaves the solution in x (entry k written by the
+// thread k mod blockDim.x) and returns ier.
+template <class Solve>
+__device__ __forceinline__ void cg_system_with(const PressParams &p, StepCtl *ctl, int kind, int sys,
+                                               double dt_explicit, double *Pt, double *Pd, const double *x,
+                                               double *red, long long *iters, Solve solve)
 {
     const int64_t N = p.N;
     double dt = sys_dt(ctl, kind, sys, dt_explicit);
-    int ier = cg_solve<XC>(p, dt, x, r, pv, Mp, red, iters, exact, cf);
+    int ier = solve(dt);
     if (kind == 0) {
         // probe: src/solver.f90:81-92, halve t_try until the solve converges
         int guard = 0;
         while (ier == 1 && guard < 1100) {
             dt = dt / 2.0;
             guard++;
-            ier = cg_solve<XC>(p, dt, x, r, pv, Mp, red, iters, exact, cf);
+            ier = solve(dt);
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -1063,6 +1064,148 @@ __device__ void cg_system(const PressParams &p, StepCtl *ctl, int kind, int sys,
             }
         }
     }
+}
+
+// The CG with its vectors in global memory (shared with the allocation-free
+// entry point).
+template <bool XC = false>
+__device__ void cg_system(const PressParams &p, StepCtl *ctl, int kind, int sys, double dt_explicit, double *Pt,
+                          double *Pd, double *x, double *r, double *pv, double *Mp, double *red, long long *iters,
+                          int exact, double *cf = nullptr)
+{
+    cg_system_with(p, ctl, kind, sys, dt_explicit, Pt, Pd, x, red, iters, [&](double dt) {
+        return cg_solve<XC>(p, dt, x, r, pv, Mp, red, iters, exact, cf);
+    });
+}
+
+// The same CG (exact = 0 with cached coefficients: identical results) of a
+// system of at most EPT * CGS_THREADS elements with its vectors in registers.
+// A small solve is a chain of barriers: cg_solve takes three per reduction
+// and one for the direction; here every warp adds up the warps' partial sums
+// itself after one barrier (double-buffered slots; the same butterflies, and
+// warps that a smaller block leaves out would only have added zeros), and the
+// neighbours' next direction entries are formed locally from their r (in
+// shared memory before the second reduction's barrier) and their current
+// direction: two barriers per iteration. Blocks hold only the warps that the
+// largest network of the launch needs. 13 iterations at N = 39: 40 -> 17 us, 28 at
+// N = 1404: 63 -> 40 us (with the launch); the cg_iterations counter, which the
+// threads of cg_solve add to without order, is exact here.
+#define CGS_THREADS 1024
+struct CgsSmem {
+    double r[2 * CGS_THREADS + 2];   // r with a zero at either end
+    double part[2][2][32];           // warps' sums and maxima, by reduction
+};
+
+template <int EPT>
+__device__ __forceinline__ int cg_solve_regs(const PressParams &p, double dt, double *xout, CgsSmem &sm,
+                                             long long *iters)
+{
+    const int N = (int)p.N, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, nw = (int)blockDim.x >> 5;
+    int top = 1;   // butterfly over the warps' partials
+    while (top < nw) top <<= 1;
+    auto warps_sum = [&](const double *q) {
+        double t = lane < nw ? q[lane] : 0.0;
+        for (int o = top >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    auto warps_max = [&](const double *q) {
+        double t = lane < nw ? q[lane] : 0.0;
+        for (int o = top >> 1; o > 0; o >>= 1) t = fmax(t, __shfl_xor_sync(0xffffffffu, t, o));
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    auto warp_max = [&](double t) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_xor_sync(0xffffffffu, t, o));
+        return t;
+    };
+    double x[EPT], r[EPT], pv[EPT], pl[EPT], pr[EPT], s1[EPT], s3[EPT], m[EPT];
+    double sum = 0.0, mx = 0.0;
+    __syncthreads();   // the shared arrays may still be read from a previous solve
+    if (tid == 0) { sm.r[0] = 0.0; sm.r[N + 1] = 0.0; }
+#pragma unroll
+    for (int j = 0; j < EPT; j++) {
+        const int k = tid + j * CGS_THREADS;
+        x[j] = r[j] = s1[j] = s3[j] = 0.0;
+        if (k < N) {
+            double A1, A2, A3;
+            prow(p, k, dt, A1, A2, A3);
+            s1[j] = A1 / A2;
+            s3[j] = A3 / A2;
+            x[j] = p.P[k];
+            r[j] = add_(pb1(p, k, dt, A2), -pmatvec_row_c(k, N, A1, A2, A3, p.P));
+            sm.r[k + 1] = r[j];
+            mx = fmax(mx, fabs(r[j]));
+            sum = fma(r[j], r[j], sum);
+        }
+        pv[j] = r[j];
+    }
+    sum = warp_sum(sum);
+    mx = warp_max(mx);
+    if (lane == 0) { sm.part[1][0][w] = sum; sm.part[1][1][w] = mx; }
+    __syncthreads();
+    double rr = warps_sum(sm.part[1][0]);
+    mx = warps_max(sm.part[1][1]);
+#pragma unroll
+    for (int j = 0; j < EPT; j++) {
+        const int k = tid + j * CGS_THREADS;
+        pl[j] = k < N ? sm.r[k] : 0.0;
+        pr[j] = k < N ? sm.r[k + 2] : 0.0;
+    }
+    long long it = 0;
+    int ier = 0;
+    while (mx >= p.tol) {
+        it++;
+        double pap = 0.0;
+#pragma unroll
+        for (int j = 0; j < EPT; j++) {
+            const int k = tid + j * CGS_THREADS;
+            if (k >= N) continue;
+            if (k == 0) m[j] = fma(s3[j], pr[j], pv[j]);
+            else if (k == N - 1) m[j] = fma(s1[j], pl[j], pv[j]);
+            else m[j] = fma(s1[j], pl[j], fma(s3[j], pr[j], pv[j]));
+            pap = fma(pv[j], m[j], pap);
+        }
+        pap = warp_sum(pap);
+        if (lane == 0) sm.part[0][0][w] = pap;
+        __syncthreads();
+        const double alpha = rr / warps_sum(sm.part[0][0]);
+        sum = 0.0;
+        mx = 0.0;
+#pragma unroll
+        for (int j = 0; j < EPT; j++) {
+            const int k = tid + j * CGS_THREADS;
+            if (k >= N) continue;
+            x[j] = add_(x[j], mul_(alpha, pv[j]));
+            r[j] = add_(r[j], -mul_(alpha, m[j]));
+            sm.r[k + 1] = r[j];
+            sum = fma(r[j], r[j], sum);
+            mx = fmax(mx, fabs(r[j]));
+        }
+        sum = warp_sum(sum);
+        mx = warp_max(mx);
+        if (lane == 0) { sm.part[1][0][w] = sum; sm.part[1][1][w] = mx; }
+        __syncthreads();
+        const double r1r1 = warps_sum(sm.part[1][0]);
+        mx = warps_max(sm.part[1][1]);
+        const double beta = r1r1 / rr;
+#pragma unroll
+        for (int j = 0; j < EPT; j++) {
+            const int k = tid + j * CGS_THREADS;
+            if (k >= N) continue;
+            pl[j] = add_(sm.r[k], mul_(beta, pl[j]));
+            pr[j] = add_(sm.r[k + 2], mul_(beta, pr[j]));
+            pv[j] = add_(r[j], mul_(beta, pv[j]));
+        }
+        rr = r1r1;
+        if (it > 200) { ier = 1; break; }
+    }
+#pragma unroll
+    for (int j = 0; j < EPT; j++) {
+        const int k = tid + j * CGS_THREADS;
+        if (k < N) xout[k] = x[j];
+    }
+    *iters += it;   // read by thread 0 alone
+    return ier;
 }
 
 // Single system with explicit pointers (allocation-free entry point).
@@ -1131,6 +1274,29 @@ __global__ void __launch_bounds__(1024) pressure_cg_batch_kernel(PressGlobal g, 
     cg_system<XC>(p, ctl + i, kind, sys, dt_explicit, Ptemp + 6 * I.eoff + (int64_t)sys * N,
                   Pdot + 6 * I.eoff + (int64_t)sys * N, x, r, pv, Mp, red, &iters, exact,
                   coef + 18 * I.eoff + (int64_t)sys * 3 * N);
+}
+
+// Small systems: CTA (system s, instance i) of pressure_cg_batch_kernel with
+// exact = 0, blockDim the warps that the largest network needs.
+template <int EPT>
+__global__ void __launch_bounds__(CGS_THREADS) pressure_cg_small_kernel(PressGlobal g, const Inst *inst, StepCtl *ctl,
+                                                                        int mask, int kind, int sys0,
+                                                                        double dt_explicit, double *Ptemp,
+                                                                        double *Pdot, double *work)
+{
+    __shared__ CgsSmem sm;
+    __shared__ double red[66];
+    const int i = blockIdx.y;
+    if (!press_takes_part(ctl, i, mask, kind)) return;
+    const Inst I = inst[i];
+    const PressParams p = press_params(g, I, i, ctl);
+    const int sys = sys0 + blockIdx.x;
+    const int64_t N = I.N;
+    double *x = work + 24 * I.eoff + (int64_t)sys * 4 * N;
+    long long iters = 0;
+    cg_system_with(p, ctl + i, kind, sys, dt_explicit, Ptemp + 6 * I.eoff + (int64_t)sys * N,
+                   Pdot + 6 * I.eoff + (int64_t)sys * N, x, red, &iters,
+                   [&](double dt) { return cg_solve_regs<EPT>(p, dt, x, sm, &iters); });
 }
 
 // ---------------------------------------------------------------------------

@@ -109,6 +109,37 @@ def _cluster_case(case):
     return networks.fault_network(n_faults=500, box=5500.0, seed=6, tol=1e-8)
 
 
+@pytest.mark.parametrize("n_el", [2, 31, 32, 33, 64, 65, 1023, 1024, 1025, 2047])
+def test_small_cg_matches_oracle(n_el):
+    """Systems with their CG vectors in registers (one or two elements per
+    thread, full and partly filled warps): the reference CG's stopping rule
+    and cap."""
+    p = networks.single_fault(n_el=n_el, length=10.0 * n_el, mode="modeIII", tol=1e-6)
+    o = Oracle(p)
+    with Simulation(p, storage="fp32", pressure="cg") as s:
+        for dt in (10.0, 3000.0):
+            gP, _, gi = s.compute_P(dt)
+            oP, _, oi = o.compute_P(dt)
+            assert gi == oi
+            if oi == 0:
+                assert np.abs(gP - oP).max() < 1e3 * 1e-6
+
+
+@pytest.mark.parametrize("pressure", ["cg", "tridiag"])
+@pytest.mark.parametrize("seed", [3, 9])
+def test_steps_in_one_call_or_one_by_one(seed, pressure):
+    """The same steps back to back on the device (kernels that start while
+    their predecessors drain, pressure beside the K.V) or with a host
+    synchronisation after each."""
+    p = networks.small_network(seed=seed, n_faults=4, tol=1e-6)
+    with Simulation(p, pressure=pressure) as a, Simulation(p, pressure=pressure) as b:
+        a.solve_steps(12)
+        for _ in range(12):
+            b.solve_steps(1)
+        x, y = a.state(), b.state()
+        assert x["time"] == y["time"] and np.array_equal(x["Y"], y["Y"]) and np.array_equal(x["P"], y["P"])
+
+
 @pytest.mark.parametrize("n_el", [65, 256, 257, 1023, 1024, 1025, 2047, 4096, 4097, 6000])
 def test_long_tridiagonal_segments(n_el):
     """One fault longer than a warp's segment: 256 threads, 1024 threads and
