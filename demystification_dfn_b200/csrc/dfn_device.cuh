@@ -996,10 +996,13 @@ __device__ int cg_solve(const PressParams &p, double dt, double *x, double *r, d
         // the next stencil reads the neighbours' pv: all updates first
         __syncthreads();
         rr = r1r1;
-        if (it > 200) { *iters += it; return 1; }
+        if (it > 200) {
+            if (tid == 0) *iters += it;
+            return 1;
+        }
         errmax = mx / p.tol;
     }
-    *iters += it;
+    if (tid == 0) *iters += it;
     return 0;
 }
 
@@ -1088,8 +1091,7 @@ __device__ void cg_system(const PressParams &p, StepCtl *ctl, int kind, int sys,
 // shared memory before the second reduction's barrier) and their current
 // direction: two barriers per iteration. Blocks hold only the warps that the
 // largest network of the launch needs. 13 iterations at N = 39: 40 -> 17 us, 28 at
-// N = 1404: 63 -> 40 us (with the launch); the cg_iterations counter, which the
-// threads of cg_solve add to without order, is exact here.
+// N = 1404: 63 -> 40 us (with the launch).
 #define CGS_THREADS 1024
 struct CgsSmem {
     double r[2 * CGS_THREADS + 2];   // r with a zero at either end
@@ -1470,7 +1472,7 @@ __device__ int cg_solve_cluster(const PressParams &p, double dt, int64_t k0, int
     // the next solve (or the output) may reuse the slots and buffers only
     // after every CTA has read this one's last partial sums
     cl.sync();
-    *iters += it;
+    if (tid == 0) *iters += it;
     return ier;
 }
 
