@@ -86,6 +86,8 @@ struct dfn_handle {
     // rows (fork after the permutation, join before the row sums)
     cudaStream_t side_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaStream_t hm_stream[2] = {nullptr, nullptr};   // wide leaves, larger whole leaves of smaller matrices
+    cudaEvent_t hm_join[2] = {nullptr, nullptr};
     cudaEvent_t ev_pfork = nullptr, ev_pjoin = nullptr;   // pressure solves beside a K.V
     cudaStream_t side_lo = nullptr;       // lowest priority: tiled pressure filling around the tensor-core GEMM
     cudaGraphExec_t graph_exec = nullptr;
@@ -272,12 +274,23 @@ static int launch_hmat(dfn_handle *h, int mask, const double *Vbase, int vmul, b
 
     // the low-rank leaves (latency-bound; the rows of the wide ones after
     // their z partials) on the side stream, issued first, beside the dense
-    // rows (bandwidth-bound) on the handle's stream
+    // rows (bandwidth-bound) on the handle's stream. Below a few waves of
+    // CTAs each of these launches is one long chain of loads that leaves the
+    // GPU idle, so the wide leaves, and in smaller matrices the larger whole
+    // leaves, get streams of their own: K.V at N = 8 400 (0.1 GB) 130 -> 104
+    // (wide) -> 72 us (both); 16 steps at N = 20 000 (0.4 GB) 24.9 -> 19.1 ->
+    // 20.8 ms, at N = 41 000 (1.2 GB) 30.0 -> 27.8 -> 27.7 ms; at N = 81 750
+    // (3.2 GB) the K.V is bound by bandwidth and the launches in sequence read
+    // better: 0.72 -> 0.78 -> 0.75 ms.
     const bool fork = (n1 > 0 || n2 > 0 || n4 > 0 || n5 > 0) && n3 > 0 && h->side_stream;
+    const bool wide_own = fork && n1 > 0 && h->kv_bytes <= (int64_t)2 << 30;
+    const bool whole_own = fork && n4 > 0 && h->kv_bytes <= (int64_t)1 << 28;
     cudaStream_t ls = fork ? h->side_stream : h->stream;
     if (fork) {
         CK(cudaEventRecord(h->ev_fork, h->stream));
         CK(cudaStreamWaitEvent(h->side_stream, h->ev_fork, 0));
+        for (int j = 0; j < 2; j++)
+            if (j == 0 ? wide_own : whole_own) CK(cudaStreamWaitEvent(h->hm_stream[j], h->ev_fork, 0));
     }
     if (n5 > 0 && h->small_form == 1) {
         if (h->store == 0)
@@ -310,15 +323,17 @@ static int launch_hmat(dfn_handle *h, int mask, const double *Vbase, int vmul, b
         CKL();
     }
     if (n4 > 0) {
+        const cudaStream_t ls4 = whole_own ? h->hm_stream[1] : ls;
         if (h->store == 0)
-            hm_lowrank_fused_kernel<double><<<(unsigned)n4, 256, 0, ls>>>(
+            hm_lowrank_fused_kernel<double><<<(unsigned)n4, 256, 0, ls4>>>(
                 h->hl4, h->hblk, h->inst, h->ctl, mask, (const double *)h->hvals, h->hxp, h->hout);
         else
-            hm_lowrank_fused_kernel<float><<<(unsigned)n4, 256, 0, ls>>>(
+            hm_lowrank_fused_kernel<float><<<(unsigned)n4, 256, 0, ls4>>>(
                 h->hl4, h->hblk, h->inst, h->ctl, mask, (const float *)h->hvals, h->hxp, h->hout);
         h->launches++;
         CKL();
     }
+    if (wide_own) ls = h->hm_stream[0];
     if (n1 > 0) {
         if (h->store == 0)
             hm_lowrank_kernel<double><<<(unsigned)n1, 256, 0, ls>>>(
@@ -362,11 +377,15 @@ static int launch_hmat(dfn_handle *h, int mask, const double *Vbase, int vmul, b
     if (fork) {
         CK(cudaEventRecord(h->ev_join, h->side_stream));
         CK(cudaStreamWaitEvent(h->stream, h->ev_join, 0));
+        for (int j = 0; j < 2; j++)
+            if (j == 0 ? wide_own : whole_own) {
+                CK(cudaEventRecord(h->hm_join[j], h->hm_stream[j]));
+                CK(cudaStreamWaitEvent(h->stream, h->hm_join[j], 0));
+            }
     }
-    hm_gather_kernel<<<blocks_of(ne, 256), 256, 0, h->stream>>>(ne, h->ncomp, h->inst_of, h->inst, h->ctl, mask,
-                                                                h->hperm, h->hsegof, h->hsegptr, h->hsegbase, h->hout,
-                                                                h->partT,
-                                                                h->partN);
+    hm_gather_kernel<<<dim3(blocks_of(ne, 256), (unsigned)h->ncomp), 256, 0, h->stream>>>(
+        ne, h->inst_of, h->inst, h->ctl, mask, h->hperm, h->hsegof, h->hsegptr, h->hsegbase, h->hout, h->partT,
+        h->partN);
     h->launches++;
     CKL();
     return DFN_OK;
@@ -1417,6 +1436,10 @@ int32_t dfn_destroy(dfn_handle *h)
     if (h->cap_stream) cudaStreamDestroy(h->cap_stream);
     if (h->side_stream) cudaStreamDestroy(h->side_stream);
     if (h->side_lo) cudaStreamDestroy(h->side_lo);
+    for (int j = 0; j < 2; j++) {
+        if (h->hm_stream[j]) cudaStreamDestroy(h->hm_stream[j]);
+        if (h->hm_join[j]) cudaEventDestroy(h->hm_join[j]);
+    }
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->ev_pfork) cudaEventDestroy(h->ev_pfork);
@@ -1822,6 +1845,10 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
         CKC(cudaStreamCreateWithPriority(&h->side_stream, cudaStreamNonBlocking, hi_pri));
         CKC(cudaStreamCreateWithPriority(&h->side_lo, cudaStreamNonBlocking, lo_pri));
         CKC(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+        for (int j = 0; j < 2 && h->hmat; j++) {
+            CKC(cudaStreamCreateWithPriority(&h->hm_stream[j], cudaStreamNonBlocking, hi_pri));
+            CKC(cudaEventCreateWithFlags(&h->hm_join[j], cudaEventDisableTiming));
+        }
         CKC(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
         CKC(cudaEventCreateWithFlags(&h->ev_pfork, cudaEventDisableTiming));
         CKC(cudaEventCreateWithFlags(&h->ev_pjoin, cudaEventDisableTiming));

@@ -970,7 +970,10 @@ __global__ void __launch_bounds__(256) hm_aca_place_kernel(const AcaLeaf *__rest
 // segment of rows in block order; a warp's rows mostly share a segment, so
 // the bases are broadcast and the slot reads coalesced), stored at the
 // original element index in the K.V result arrays (partials with one chunk).
-__global__ void hm_gather_kernel(int64_t Ntot, int ncomp, const int *__restrict__ inst_of,
+// grid (rows, components). A row is a chain of dozens of slot reads and
+// nothing else, so a thread per component and eight slots in flight.
+// K.V 0.741 -> 0.725 ms at N = 81 750, 0.400 -> 0.390 ms for 24 networks.
+__global__ void hm_gather_kernel(int64_t Ntot, const int *__restrict__ inst_of,
                                  const Inst *__restrict__ inst, const StepCtl *__restrict__ ctl, int mask,
                                  const int *__restrict__ perm, const int32_t *__restrict__ segof,
                                  const int64_t *__restrict__ segptr, const int64_t *__restrict__ segbase,
@@ -978,14 +981,23 @@ __global__ void hm_gather_kernel(int64_t Ntot, int ncomp, const int *__restrict_
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= Ntot) return;
+    const int c = blockIdx.y;
     const int i = inst_of[e];
     if (!takes_part(ctl, i, mask)) return;
     const Inst &I = inst[i];
     const int64_t orig = perm[e];   // perm[eoff + pos], a network-local index
-    for (int c = 0; c < ncomp; c++) {
-        const int sg = segof[(int64_t)c * Ntot + e];
-        double s = 0.0;
-        for (int64_t j = segptr[sg]; j < segptr[sg + 1]; j++) s += out[segbase[j] + e];
-        (c == 0 ? partT : partN)[I.poff + orig] = s;
+    const int sg = segof[(int64_t)c * Ntot + e];
+    const int64_t *base = segbase + segptr[sg];
+    const double *oe = out + e;
+    double s = 0.0;
+    int n = (int)(segptr[sg + 1] - segptr[sg]);
+    for (; n >= 8; n -= 8, base += 8) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[q] = oe[base[q]];
+#pragma unroll
+        for (int q = 0; q < 8; q++) s += v[q];
     }
+    for (int q = 0; q < n; q++) s += oe[base[q]];
+    (c == 0 ? partT : partN)[I.poff + orig] = s;
 }
