@@ -320,13 +320,19 @@ __global__ void __launch_bounds__(256) hm_lowrank_fused_kernel(const int *__rest
 // the rank in order, as in hm_lowrank_fused_kernel), written to the leaf's
 // output slots. Leaves qualify when their factors take at most
 // HM_WARP_LEAF_BYTES and their B^T rows at most 32 * HM_WARP_XV vectors.
-// These leaves are a few KB each and latency-bound: a SM holds the loads of
-// dozens of them in flight, against 8 with one CTA per leaf. The kernel is
-// held to 40 registers (12 CTAs of four warps per SM, a few spills to L1)
-// and the dense-row kernel to 48 (five CTAs of 256): K.V 0.840 -> 0.823 ms
-// at N = 81 750 (8 CTAs and 64 registers each before).
+// These leaves are a few KB each and latency-bound: what counts is how many
+// loads an SM has in flight. Four rows of B^T per pass, all loaded before
+// their products, with a reduction that hands halves of the rows to the
+// partner lane (5 shuffles instead of 16 for four rows), at 64 registers
+// (8 CTAs of four warps) beat one row per pass at 40 registers (12 CTAs):
+// K.V 0.725 -> 0.690 ms at N = 81 750, 0.381 -> 0.357 ms for 24 networks;
+// two rows at 40 registers 0.703 and 0.363, four rows at 48 and 40 registers
+// 0.700 / 0.697 and 0.363 / 0.359, eight rows 0.701 and 0.366. The dense-row
+// kernel is held to 48 registers (five CTAs of 256).
 constexpr int HM_WARP_LEAF_BYTES = 32 * 1024;
 constexpr int HM_WARP_XV = 2;
+constexpr int HM_WARP_NB = 4;     // rows per group of lanes and pass
+constexpr int HM_WARP_CTAS = 8;   // resident CTAs per SM (64 registers)
 
 struct HLeafW {
     int64_t aoff;     // A^T offset (values); B^T follows at aoff + rank * lda
@@ -378,56 +384,26 @@ __device__ __forceinline__ void hm_warp_az(const HLeafW &d, const T *__restrict_
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(128, 12) hm_lowrank_warp_kernel(const HLeafW *__restrict__ leaves, int64_t n,
-                                                                  const StepCtl *__restrict__ ctl, int mask,
-                                                                  const T *__restrict__ vals,
-                                                                  const double *__restrict__ xp,
-                                                                  double *__restrict__ out)
+// Sum over a group of g lanes (a power of two, g >= NB) of NB values each:
+// the first log2(NB) butterfly steps hand one half of the values to the
+// partner and keep the other, so value j ends in the lanes whose top bits
+// within the group are j. The additions are those of NB plain butterflies.
+template <int NB>
+__device__ __forceinline__ double hm_reduce_scatter(double *acc, int lane, int g)
 {
-    using VT = typename HVec<T>::V;
-    constexpr int W = HVec<T>::W;
-    __shared__ double zs[4][hmat::kMaxRank];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t k = (int64_t)blockIdx.x * 4 + warp;
-    if (k >= n) return;   // warp-uniform; the kernel has no block barrier
-    const HLeafW d = leaves[k];
-    if (!takes_part(ctl, d.inst, mask)) return;
-    const int rank = d.rank, nv = d.ld / W;
-    int g = 1;
-    while (g < nv && g < 32) g <<= 1;
-    const int sub = lane / g, v0 = lane % g, rp = 32 / g;
-    double xv[HM_WARP_XV][W];
+    int o = g >> 1;
 #pragma unroll
-    for (int m = 0; m < HM_WARP_XV; m++) {
-        const int v = v0 + m * g;
+    for (int n = NB >> 1; n > 0; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
 #pragma unroll
-        for (int c = 0; c < W; c++) xv[m][c] = (v < nv) ? __ldg(xp + d.xoff + v * W + c) : 0.0;
-    }
-    const T *A = vals + d.aoff;
-    const VT *Bt = reinterpret_cast<const VT *>(A + (int64_t)rank * d.lda);
-    double *z = zs[warp];
-#pragma unroll 4
-    for (int q0 = 0; q0 < rank; q0 += rp) {
-        const int q = q0 + sub;
-        double acc = 0.0;
-        if (q < rank) {
-#pragma unroll
-            for (int m = 0; m < HM_WARP_XV; m++) {
-                const int v = v0 + m * g;
-                if (v < nv) {
-                    double f[W];
-                    HVec<T>::unpack(Bt[(int64_t)q * nv + v], f);
-#pragma unroll
-                    for (int c = 0; c < W; c++) acc = fma(f[c], xv[m][c], acc);
-                }
-            }
+        for (int j = 0; j < n; j++) {
+            const double give = up ? acc[j] : acc[j + n], keep = up ? acc[j + n] : acc[j];
+            acc[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
         }
-        for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (v0 == 0 && q < rank) z[q] = acc;
     }
-    __syncwarp();
-    hm_warp_az<T>(d, A, z, out, lane);
+    double t = acc[0];
+    for (; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
 }
 
 template <typename T>
@@ -439,9 +415,8 @@ __device__ __forceinline__ void hm_lowrank_warp_leaf(const HLeafW &d, const T *_
     constexpr int W = HVec<T>::W;
     const int lane = threadIdx.x & 31;
     const int rank = d.rank, nv = d.ld / W;
-    int g = 1;
-    while (g < nv && g < 32) g <<= 1;
-    const int sub = lane / g, v0 = lane % g, rp = 32 / g;
+    const int lg = nv >= 32 ? 5 : (nv <= 1 ? 0 : 32 - __clz(nv - 1));
+    const int g = 1 << lg, sub = lane >> lg, v0 = lane & (g - 1), rp = 32 >> lg;
     double xv[HM_WARP_XV][W];
 #pragma unroll
     for (int m = 0; m < HM_WARP_XV; m++) {
@@ -451,35 +426,73 @@ __device__ __forceinline__ void hm_lowrank_warp_leaf(const HLeafW &d, const T *_
     }
     const T *A = vals + d.aoff;
     const VT *Bt = reinterpret_cast<const VT *>(A + (int64_t)rank * d.lda);
-#pragma unroll 4
-    for (int q0 = 0; q0 < rank; q0 += rp) {
-        const int q = q0 + sub;
-        double acc = 0.0;
-        if (q < rank) {
+    const VT zero{};
+    int q0 = 0;
+    if (g >= HM_WARP_NB) {
+        // HM_WARP_NB rows per group of lanes and pass
+        for (; q0 < rank; q0 += HM_WARP_NB * rp) {
+            const VT *row = Bt + (q0 + sub) * nv + v0;   // a leaf holds at most 32 KiB
+            double acc[HM_WARP_NB];
+#pragma unroll
+            for (int j = 0; j < HM_WARP_NB; j++) acc[j] = 0.0;
 #pragma unroll
             for (int m = 0; m < HM_WARP_XV; m++) {
-                const int v = v0 + m * g;
-                if (v < nv) {
-                    double f[W];
-                    HVec<T>::unpack(Bt[(int64_t)q * nv + v], f);
+                if (m * g >= nv) break;   // warp-uniform
+                VT f[HM_WARP_NB];
 #pragma unroll
-                    for (int c = 0; c < W; c++) acc = fma(f[c], xv[m][c], acc);
+                for (int j = 0; j < HM_WARP_NB; j++)
+                    f[j] = (q0 + sub + j * rp < rank && v0 + m * g < nv) ? row[j * rp * nv + m * g] : zero;
+#pragma unroll
+                for (int j = 0; j < HM_WARP_NB; j++) {
+                    double u[W];
+                    HVec<T>::unpack(f[j], u);
+#pragma unroll
+                    for (int c = 0; c < W; c++) acc[j] = fma(u[c], xv[m][c], acc[j]);
                 }
             }
+            const double t = hm_reduce_scatter<HM_WARP_NB>(acc, lane, g);
+            const int per = g / HM_WARP_NB;   // lanes that hold the same row's sum
+            const int q = q0 + sub + (v0 / per) * rp;
+            if ((v0 & (per - 1)) == 0 && q < rank) z[q] = t;
+        }
+    }
+    for (; q0 < rank; q0 += rp) {
+        const int q = q0 + sub;
+        double acc = 0.0;
+        if (q < rank && v0 < nv) {
+            double u[W];
+            HVec<T>::unpack(Bt[q * nv + v0], u);
+#pragma unroll
+            for (int c = 0; c < W; c++) acc = fma(u[c], xv[0][c], acc);
         }
         for (int o = g >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (v0 == 0 && q < rank) z[q] = acc;
     }
     __syncwarp();
     hm_warp_az<T>(d, A, z, out, lane);
-    __syncwarp();   // z is rewritten by the warp's next leaf
+}
+
+template <typename T>
+__global__ void __launch_bounds__(128, HM_WARP_CTAS) hm_lowrank_warp_kernel(const HLeafW *__restrict__ leaves, int64_t n,
+                                                                            const StepCtl *__restrict__ ctl, int mask,
+                                                                            const T *__restrict__ vals,
+                                                                            const double *__restrict__ xp,
+                                                                            double *__restrict__ out)
+{
+    __shared__ double zs[4][hmat::kMaxRank];
+    const int warp = threadIdx.x >> 5;
+    const int64_t k = (int64_t)blockIdx.x * 4 + warp;
+    if (k >= n) return;   // warp-uniform; the kernel has no block barrier
+    const HLeafW d = leaves[k];
+    if (!takes_part(ctl, d.inst, mask)) return;
+    hm_lowrank_warp_leaf<T>(d, vals, xp, out, zs[warp]);
 }
 
 // The same leaves on a persistent grid: warp w of CTA c takes leaves
 // 4c + w, 4c + w + 4 gridDim.x, ... (each leaf's arithmetic is that of
 // hm_lowrank_warp_kernel).
 template <typename T>
-__global__ void __launch_bounds__(128, 12) hm_lowrank_warp_persistent_kernel(const HLeafW *__restrict__ leaves, int64_t n,
+__global__ void __launch_bounds__(128, HM_WARP_CTAS) hm_lowrank_warp_persistent_kernel(const HLeafW *__restrict__ leaves, int64_t n,
                                                                   const StepCtl *__restrict__ ctl, int mask,
                                                                   const T *__restrict__ vals,
                                                                   const double *__restrict__ xp,
@@ -491,6 +504,7 @@ __global__ void __launch_bounds__(128, 12) hm_lowrank_warp_persistent_kernel(con
         const HLeafW d = leaves[k];
         if (!takes_part(ctl, d.inst, mask)) continue;   // warp-uniform; the kernel has no block barrier
         hm_lowrank_warp_leaf<T>(d, vals, xp, out, zs[warp]);
+        __syncwarp();   // z is rewritten by the warp's next leaf
     }
 }
 

@@ -173,3 +173,21 @@ def test_loaded_network_event_onset_hmatrix():
     assert kg is not None and kf is not None
     assert abs(tg - to) <= 1e-3 * to
     assert abs(tf - tg) <= 1e-4 * tg
+
+
+@pytest.mark.parametrize("leaf", [2, 4, 7, 16, 40, 130, 250])
+@pytest.mark.parametrize("storage", ["fp64", "fp32"])
+@pytest.mark.parametrize("mode", ["modeII", "modeIII"])
+def test_hmat_small_leaf_shapes(leaf, storage, mode):
+    """Whole low-rank leaves of every shape the one-warp kernel takes (rows of
+    one to 64 vectors of 16 bytes, ranks that fill a pass or not): within
+    summation order of one CTA per leaf, FP64 sums of the same factors."""
+    p = networks.fault_network(n_faults=60, box=3000.0, seed=leaf, kernel="hmatrix", mode=mode)
+    with Simulation(p, storage=storage, pressure="tridiag", hmat_leaf=leaf, hmat_eta=2.0, hmat_eps=1e-6) as s:
+        v = np.random.default_rng(leaf).normal(size=s.N)
+        warp = s.kernel(v)
+        s.set_hmat_small_leaves("cta")
+        cta = s.kernel(v)
+        scale = np.abs(cta[0]).max()
+        for a, b in zip(warp, cta):
+            assert np.abs(a - b).max() <= 1e-12 * scale
