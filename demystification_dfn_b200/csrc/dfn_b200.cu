@@ -2743,52 +2743,47 @@ int32_t dfn_record_read(dfn_handle *h, float *x, float *t, int64_t max, int64_t 
 }
 
 // Gradient (and optionally an Adam step) over samples [0, n) of device
-// arrays in batches; returns the summed squared error.
+// arrays; the summed squared error goes to *dls. Two launches, in order on s.
 static int mlp_pass(const float *dX, const float *dT, int64_t n, int64_t n_total, float *dW, float *dm, float *dv,
-                    float *dg, float *dgp, float *dlp, float *dls, int step, float lr, float *loss_sum,
-                    cudaStream_t s)
+                    float *dg, float *dgp, float *dlp, float *dls, int step, float lr, cudaStream_t s)
 {
     const int nblk = (int)((n + MLP_SB - 1) / MLP_SB);
-    const size_t smem = sizeof(MlpSmem);
-    CK(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    mlp_grad_kernel<<<nblk, 256, smem, s>>>(dX, dT, n, n_total, dW, dgp, dlp);
-    CKL();
-    mlp_reduce_adam_kernel<<<(MLP_NPAR + 255) / 256, 256, 0, s>>>(dgp, nblk, dW, dm, dv, dg, step, lr);
-    CKL();
-    sum_kernel<<<1, 32, 0, s>>>(dlp, nblk, dls);
-    CKL();
-    float l = 0.0f;
-    CK(cudaMemcpyAsync(&l, dls, sizeof(float), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    *loss_sum = l;
+    CK(launch_pdl(mlp_grad_kernel, (unsigned)nblk, 256, sizeof(MlpSmem), s, dX, dT, n, n_total, (const float *)dW, dgp,
+                  dlp));
+    CK(launch_pdl(mlp_reduce_adam_kernel, blocks_of(MLP_NPAR + 1, 128), 128, 0, s, (const float *)dgp,
+                  (const float *)dlp, nblk, dW, dm, dv, dg, dls, step, lr));
     return DFN_OK;
 }
 
+// Device arrays of a training call, in one allocation: n samples, minibatches
+// of `batch`, a loss per minibatch.
 struct MlpBuffers {
+    float *base = nullptr;
     float *X = nullptr, *T = nullptr, *W = nullptr, *m = nullptr, *v = nullptr, *g = nullptr, *gp = nullptr,
           *lp = nullptr, *ls = nullptr;
     ~MlpBuffers()
     {
-        float *p[] = {X, T, W, m, v, g, gp, lp, ls};
-        for (float *q : p)
-            if (q) cudaFree(q);
+        if (base) cudaFree(base);
     }
 };
 
-static int mlp_alloc(MlpBuffers &b, int64_t n, int64_t batch)
+static int mlp_alloc(MlpBuffers &b, int64_t n, int64_t batch, int64_t losses)
 {
-    const int64_t nblk = (batch + MLP_SB - 1) / MLP_SB;
-    CK(cudaMalloc((void **)&b.X, sizeof(float) * MLP_IN * std::max<int64_t>(n, 1)));
-    CK(cudaMalloc((void **)&b.T, sizeof(float) * std::max<int64_t>(n, 1)));
-    CK(cudaMalloc((void **)&b.W, sizeof(float) * MLP_NPAR));
-    CK(cudaMalloc((void **)&b.m, sizeof(float) * MLP_NPAR));
-    CK(cudaMalloc((void **)&b.v, sizeof(float) * MLP_NPAR));
-    CK(cudaMalloc((void **)&b.g, sizeof(float) * MLP_NPAR));
-    CK(cudaMalloc((void **)&b.gp, sizeof(float) * MLP_NPAR * nblk));
-    CK(cudaMalloc((void **)&b.lp, sizeof(float) * nblk));
-    CK(cudaMalloc((void **)&b.ls, sizeof(float)));
-    CK(cudaMemset(b.m, 0, sizeof(float) * MLP_NPAR));
-    CK(cudaMemset(b.v, 0, sizeof(float) * MLP_NPAR));
+    const int64_t nblk = (std::min(batch, n) + MLP_SB - 1) / MLP_SB;
+    const int64_t par = (MLP_NPAR + 3) / 4 * 4;
+    int64_t at = 0;
+    auto take = [&](int64_t count) {
+        const int64_t o = at;
+        at += (count + 3) / 4 * 4;
+        return o;
+    };
+    const int64_t m = take(par), v = take(par), W = take(par), g = take(par), X = take(MLP_IN * n), T = take(n),
+                  gp = take(MLP_NPAR * nblk), lp = take(nblk), ls = take(losses);
+    CK(cudaMalloc((void **)&b.base, sizeof(float) * at));
+    b.m = b.base + m; b.v = b.base + v; b.W = b.base + W; b.g = b.base + g; b.X = b.base + X; b.T = b.base + T;
+    b.gp = b.base + gp; b.lp = b.base + lp; b.ls = b.base + ls;
+    CK(cudaMemsetAsync(b.m, 0, sizeof(float) * 2 * par, nullptr));   // m and v
+    CK(cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem)));
     return DFN_OK;
 }
 
@@ -2796,12 +2791,13 @@ int32_t dfn_mlp_loss_grad(const float *x, const float *t, int64_t n, const float
 {
     if (!x || !t || n < 1 || !weights || !loss || !grad) return DFN_ERR_ARG;
     MlpBuffers b;
-    TRY(mlp_alloc(b, n, n));
+    TRY(mlp_alloc(b, n, n, 1));
     CK(cudaMemcpy(b.X, x, sizeof(float) * MLP_IN * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.T, t, sizeof(float) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.W, weights, sizeof(float) * MLP_NPAR, cudaMemcpyHostToDevice));
+    TRY(mlp_pass(b.X, b.T, n, n, b.W, b.m, b.v, b.g, b.gp, b.lp, b.ls, 1, 0.0f, nullptr));
     float ls = 0.0f;
-    TRY(mlp_pass(b.X, b.T, n, n, b.W, b.m, b.v, b.g, b.gp, b.lp, b.ls, 1, 0.0f, &ls, nullptr));
+    CK(cudaMemcpy(&ls, b.ls, sizeof(float), cudaMemcpyDeviceToHost));
     *loss = ls / (float)n;
     CK(cudaMemcpy(grad, b.g, sizeof(float) * MLP_NPAR, cudaMemcpyDeviceToHost));
     return DFN_OK;
@@ -2811,9 +2807,7 @@ int32_t dfn_mlp_infer(const float *x, int64_t n, const float *weights, float *y)
 {
     if (!x || n < 1 || !weights || !y) return DFN_ERR_ARG;
     MlpBuffers b;
-    CK(cudaMalloc((void **)&b.X, sizeof(float) * MLP_IN * n));
-    CK(cudaMalloc((void **)&b.T, sizeof(float) * n));
-    CK(cudaMalloc((void **)&b.W, sizeof(float) * MLP_NPAR));
+    TRY(mlp_alloc(b, n, 1, 1));
     CK(cudaMemcpy(b.X, x, sizeof(float) * MLP_IN * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.W, weights, sizeof(float) * MLP_NPAR, cudaMemcpyHostToDevice));
     mlp_infer_kernel<<<(unsigned)((n + 255) / 256), 256, sizeof(MlpTC)>>>(b.X, n, b.W, b.T);
@@ -2840,23 +2834,32 @@ int32_t dfn_mlp_train(const float *x, const float *t, int64_t n, float *weights,
         for (int q = 0; q < MLP_IN; q++) xs[(size_t)i * MLP_IN + q] = x[order[i] * MLP_IN + q];
         ts[i] = t[order[i]];
     }
+    const int64_t nb = (n + batch - 1) / batch;   // minibatches per epoch
     MlpBuffers b;
-    TRY(mlp_alloc(b, n, batch));
+    TRY(mlp_alloc(b, n, batch, 2 * nb));
     CK(cudaMemcpy(b.X, xs.data(), sizeof(float) * xs.size(), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.T, ts.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(b.W, weights, sizeof(float) * MLP_NPAR, cudaMemcpyHostToDevice));
+    // the launches of all epochs in a row; the minibatch losses of the first
+    // and of the last one are kept
     int step = 0;
     for (int ep = 0; ep < epochs; ep++) {
-        double esum = 0.0;
-        for (int64_t s0 = 0; s0 < n; s0 += batch) {
+        float *ls = b.ls + (ep == 0 ? 0 : nb);
+        for (int64_t s0 = 0; s0 < n; s0 += batch, ls++) {
             const int64_t m = std::min<int64_t>(batch, n - s0);
-            float ls = 0.0f;
-            TRY(mlp_pass(b.X + s0 * MLP_IN, b.T + s0, m, m, b.W, b.m, b.v, nullptr, b.gp, b.lp, b.ls, ++step, lr,
-                         &ls, nullptr));
-            esum += ls;
+            TRY(mlp_pass(b.X + s0 * MLP_IN, b.T + s0, m, m, b.W, b.m, b.v, nullptr, b.gp, b.lp, ls, ++step, lr,
+                         nullptr));
         }
-        if (loss && ep == 0) loss[0] = (float)(esum / n);
-        if (loss && ep == epochs - 1) loss[1] = (float)(esum / n);
+    }
+    if (loss) {
+        std::vector<float> ls(2 * nb);
+        CK(cudaMemcpy(ls.data(), b.ls, sizeof(float) * (epochs > 1 ? 2 : 1) * nb, cudaMemcpyDeviceToHost));
+        for (int e = 0; e < 2; e++) {
+            const float *l = ls.data() + (epochs > 1 ? e * nb : 0);
+            double esum = 0.0;
+            for (int64_t i = 0; i < nb; i++) esum += l[i];
+            loss[e] = (float)(esum / n);
+        }
     }
     CK(cudaMemcpy(weights, b.W, sizeof(float) * MLP_NPAR, cudaMemcpyDeviceToHost));
     return DFN_OK;

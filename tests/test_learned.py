@@ -27,6 +27,19 @@ def test_mlp_oracle_gradient_matches_finite_differences():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 545])
+def test_gpu_mlp_gradient_ragged_blocks(n):
+    """Blocks of 32 samples and sixteens of block partials, full or not; the
+    same tolerances as for 1000 samples."""
+    x, t = _samples(n, 3)
+    w = learned.init_weights(4)
+    loss, g = learned.loss_grad(x, t, w)
+    ol, og = mlp_oracle.loss_grad(w, x, t)
+    assert abs(loss - ol) <= 1e-5 * abs(ol)
+    assert np.abs(g - og).max() <= 1e-4 * np.abs(og).max()
+
+
+@pytest.mark.gpu
 def test_gpu_mlp_loss_and_gradient_match_oracle():
     x, t = _samples(1000, 3)
     w = learned.init_weights(4)
