@@ -478,16 +478,43 @@ __device__ __forceinline__ void tma_bulk_g2s(void *dst, const void *src, uint32_
                  : "memory");
 }
 
+// The same copy under an L2 eviction policy.
+__device__ __forceinline__ void tma_bulk_g2s_hint(void *dst, const void *src, uint32_t bytes, uint64_t *bar,
+                                                  uint64_t policy)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+                 "[%0], [%1], %2, [%3], %4;" ::"r"(smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+                 : "memory");
+}
+__device__ __forceinline__ uint64_t l2_policy_last()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ uint64_t l2_policy_first()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
 // TMA bulk-copy variant of the same tiling: one producer warp streams the
 // 4 KiB row-chunks of the tile with cp.async.bulk into a 16-stage ring of
 // shared memory completed on mbarriers; eight consumer warps read the stages
 // with 128-bit shared loads. Rows of the tile go to consumer warps
 // round-robin, one stage per row (stage s is always read by warp s % 8).
+// The matrices are read over and over, K.V after K.V, and least-recently-used
+// replacement keeps nothing of what is larger than L2: the copies of the
+// first keep_tiles tiles stay in L2 (evict_last), the others pass through it
+// (evict_first), also past the vectors that the stage kernel reads.
 template <int MODE, int STORE>
 __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     gemv_tma_kernel(const int4 *__restrict__ tiles, const Inst *__restrict__ inst, const StepCtl *ctl,
                     int mask, const uint4 *__restrict__ Kbase, const double *Vbase, int vmul,
-                    double *__restrict__ partT, double *__restrict__ partN, int wait_polls, int *err_flag)
+                    double *__restrict__ partT, double *__restrict__ partN, int wait_polls, int *err_flag,
+                    int64_t keep_tiles)
 {
     constexpr int BPC = KFmt<MODE, STORE>::BPC;
     constexpr int CPV = 16 / BPC;
@@ -532,6 +559,7 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
         // producer: one elected lane issues the bulk copies (it reads nothing
         // that a kernel writes, so it does not wait for the previous one)
         if (lane == 0) {
+            const uint64_t policy = (int64_t)blockIdx.x < keep_tiles ? l2_policy_last() : l2_policy_first();
             int i = 0;
             for (; i < nrows; i++) {
                 int s = i % TMA_STAGES;
@@ -540,8 +568,8 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
                     break;
                 }
                 mbar_expect_tx(&full[s], GEMV_CHUNK_BYTES);
-                tma_bulk_g2s(stage + s * (GEMV_CHUNK_BYTES / 16), K + (r0 + i) * row_bytes + c * GEMV_CHUNK_BYTES,
-                             GEMV_CHUNK_BYTES, &full[s]);
+                tma_bulk_g2s_hint(stage + s * (GEMV_CHUNK_BYTES / 16), K + (r0 + i) * row_bytes + c * GEMV_CHUNK_BYTES,
+                                  GEMV_CHUNK_BYTES, &full[s], policy);
             }
             issued_s = i;
         }
