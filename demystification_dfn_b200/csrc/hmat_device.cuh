@@ -327,7 +327,11 @@ __global__ void __launch_bounds__(256) hm_lowrank_fused_kernel(const int *__rest
 // (8 CTAs of four warps) beat one row per pass at 40 registers (12 CTAs):
 // K.V 0.725 -> 0.690 ms at N = 81 750, 0.381 -> 0.357 ms for 24 networks;
 // two rows at 40 registers 0.703 and 0.363, four rows at 48 and 40 registers
-// 0.700 / 0.697 and 0.363 / 0.359, eight rows 0.701 and 0.366. The dense-row
+// 0.700 / 0.697 and 0.363 / 0.359, eight rows 0.701 and 0.366. The factors
+// are read as a stream (evict-first), which leaves L1 and L2 to x, z and the
+// slots: 0.697 -> 0.688 ms, 0.363 -> 0.355 ms, N = 8 400 70 -> 57 us; the same
+// in the kernels of the larger leaves costs them 6 % at N = 81 750, and the
+// dense rows gain nothing. The dense-row
 // kernel is held to 48 registers (five CTAs of 256).
 constexpr int HM_WARP_LEAF_BYTES = 32 * 1024;
 constexpr int HM_WARP_XV = 2;
@@ -367,7 +371,7 @@ __device__ __forceinline__ void hm_warp_az(const HLeafW &d, const T *__restrict_
 #pragma unroll 4
             for (int q = qg; q < d.rank; q += hq) {
                 double a[W];
-                HVec<T>::unpack(Av[(int64_t)q * avl + rv], a);
+                HVec<T>::unpack(__ldcs(Av + (int64_t)q * avl + rv), a);
                 const double zq = z[q];
 #pragma unroll
                 for (int c = 0; c < W; c++) acc[c] = fma(a[c], zq, acc[c]);
@@ -441,7 +445,7 @@ __device__ __forceinline__ void hm_lowrank_warp_leaf(const HLeafW &d, const T *_
                 VT f[HM_WARP_NB];
 #pragma unroll
                 for (int j = 0; j < HM_WARP_NB; j++)
-                    f[j] = (q0 + sub + j * rp < rank && v0 + m * g < nv) ? row[j * rp * nv + m * g] : zero;
+                    f[j] = (q0 + sub + j * rp < rank && v0 + m * g < nv) ? __ldcs(row + j * rp * nv + m * g) : zero;
 #pragma unroll
                 for (int j = 0; j < HM_WARP_NB; j++) {
                     double u[W];
