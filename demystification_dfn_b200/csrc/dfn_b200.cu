@@ -643,8 +643,10 @@ static ElemParams elem_params(dfn_handle *h)
 // Pressure solves beside the K.V that follows them (they depend only on the
 // stage times, not on the stage state); the stage kernel that reads them
 // waits for the join. Returns the stream: the high-priority one for the CG on
-// a few thread-block clusters or CTAs (at most half the SMs: placed first, the
-// K.V streams on the others) and for a few long tridiagonal segments, the lowest-priority one for the tiled tridiagonal
+// a few thread-block clusters (at most three fifths of the SMs: placed first,
+// the K.V streams on the others; at N = 81 750, 80 CTAs for 0.39 ms beside a
+// K.V of 0.69 ms, 8 steps 56.5 -> 55.6 ms) or CTAs and for a few long
+// tridiagonal segments (at most half the SMs), the lowest-priority one for the tiled tridiagonal
 // solve of a tensor-core batch (one tile CTA fits beside each persistent GEMM
 // CTA; issued after the GEMM, so that the GEMM's CTAs are placed first and the
 // tiles fill around them), or none (in line). The fork event is recorded
@@ -661,7 +663,7 @@ static cudaStream_t pressure_beside(dfn_handle *h, int nsys, int ninst)
         return (int64_t)nsys * ninst <= h->sms / 2 ? h->side_stream : nullptr;   // a CTA each
     if (h->pressure != DFN_PRESSURE_CG || h->pcl <= 0 || h->pcl_mode == 0 || h->pcl_mode == 2) return nullptr;
     if (h->pcl_mode < 0 && (int64_t)nsys * ninst > h->pcl_max) return nullptr;
-    return ((int64_t)nsys * ninst * h->pcl <= h->sms / 2) ? h->side_stream : nullptr;
+    return ((int64_t)nsys * ninst * h->pcl <= 3 * h->sms / 5) ? h->side_stream : nullptr;
 }
 
 static int launch_pressure_side(dfn_handle *h, cudaStream_t side, int mask, int kind, int sys0, int nsys, int ninst)

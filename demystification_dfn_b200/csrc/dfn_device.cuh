@@ -1367,27 +1367,48 @@ __host__ __device__ constexpr size_t pcl_smem_bytes(int n, bool lean)
 
 namespace cgrp = cooperative_groups;
 
-// Sum over the cluster: CTA tree sum, the CTA's partial into slot, cluster
-// barrier, then each warp sums the CL partials (bitwise the same result in
-// every lane, warp and CTA).
+// Sum over the cluster: warp sums into red, CTA barrier, warp 0 adds them and
+// puts the CTA's partial into slot, cluster barrier, then each warp sums the
+// CL partials (bitwise the same result in every lane, warp and CTA; the
+// additions of block_sum). The other warps go straight to the cluster barrier,
+// so a reduction costs one CTA barrier where block_sum has three; red and slot
+// may be written again only after another barrier of the CTA, which the two
+// alternating reductions of an iteration (with slots and red of their own)
+// give each other.
 __device__ __forceinline__ double cluster_sum(double v, double *red, double *slot)
 {
     cgrp::cluster_group cl = cgrp::this_cluster();
-    v = block_sum(v, red);
-    if (threadIdx.x == 0) *slot = v;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    v = warp_sum(v);
+    if (lane == 0) red[w] = v;
+    __syncthreads();
+    if (w == 0) {
+        const double t = warp_sum((lane < (int)(blockDim.x >> 5)) ? red[lane] : 0.0);
+        if (lane == 0) *slot = t;
+    }
     cl.sync();
-    const int lane = threadIdx.x & 31;
     double t = (lane < (int)cl.num_blocks()) ? *cl.map_shared_rank(slot, lane) : 0.0;
     return warp_sum(t);
 }
-// Sum of a and max of b over the cluster (slot: 2 doubles).
+// Sum of a and max of b over the cluster (red: 64 doubles, slot: 2 doubles).
 __device__ __forceinline__ void cluster_sum_max(double a, double b, double *red, double *slot, double &sa, double &mb)
 {
     cgrp::cluster_group cl = cgrp::this_cluster();
-    block_sum_max(a, b, red, sa, mb);
-    if (threadIdx.x == 0) { slot[0] = sa; slot[1] = mb; }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    a = warp_sum(a);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
+    if (lane == 0) { red[w] = a; red[32 + w] = b; }
+    __syncthreads();
+    if (w == 0) {
+        const bool on = lane < (int)(blockDim.x >> 5);
+        const double t = warp_sum(on ? red[lane] : 0.0);
+        double u = on ? red[32 + lane] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) u = fmax(u, __shfl_xor_sync(0xffffffffu, u, o));
+        if (lane == 0) { slot[0] = t; slot[1] = u; }
+    }
     cl.sync();
-    const int lane = threadIdx.x & 31;
     const bool on = lane < (int)cl.num_blocks();
     double t = on ? cl.map_shared_rank(slot, lane)[0] : 0.0;
     double u = on ? cl.map_shared_rank(slot, lane)[1] : 0.0;
@@ -1471,7 +1492,7 @@ __device__ int cg_solve_cluster(const PressParams &p, double dt, int64_t k0, int
             if (v.Mp) v.Mp[j] = m;
             lpap += pc[j + 1] * m;
         }
-        const double pap = cluster_sum(lpap, red, v.slot + 2);
+        const double pap = cluster_sum(lpap, red + 64, v.slot + 2);
         const double alpha = rr / pap;
         double lr1 = 0.0, lm = 0.0;
         for (int j = tid; j < nk; j += nt) {
@@ -1519,7 +1540,7 @@ __global__ void __launch_bounds__(PCL_THREADS, 1)
                                double *coef)
 {
     extern __shared__ __align__(16) double pcl_sm[];
-    __shared__ double red[66];
+    __shared__ double red[96];   // 64 for sum and max, 32 for sums
     __shared__ long long iters;
     cgrp::cluster_group cl = cgrp::this_cluster();
     const int ncl = (int)cl.num_blocks(), rank = (int)cl.block_rank();
