@@ -275,8 +275,8 @@ static int launch_hmat(dfn_handle *h, int mask, const double *Vbase, int vmul, b
     const int64_t n3 = only0 ? h->hn3_0 : h->hn3, n4 = only0 ? h->hn4_0 : h->hn4;
     const int64_t n5 = only0 ? h->hn5_0 : h->hn5;
     const int64_t ne = only0 ? h->hinst[0].N : h->Ntot;
-    hm_permute_kernel<<<blocks_of(ne, 256), 256, 0, h->stream>>>(ne, h->inst_of, h->inst, h->ctl, mask, h->hperm,
-                                                                 Vbase, vmul, h->hxp);
+    CK(launch_pdl(hm_permute_kernel, blocks_of(ne, 256), 256, 0, h->stream, ne, h->inst_of, h->inst, h->ctl, mask,
+                  h->hperm, Vbase, vmul, h->hxp));
     h->launches++;
     CKL();
 

@@ -59,10 +59,11 @@ template <> struct HVec<double> {
 
 // xp[eoff + pos] = x of network i at its element perm[pos]
 __global__ void hm_permute_kernel(int64_t Ntot, const int *__restrict__ inst_of, const Inst *__restrict__ inst,
-                                  const StepCtl *__restrict__ ctl, int mask, const int *__restrict__ perm,
-                                  const double *__restrict__ Vbase, int vmul, double *__restrict__ xp)
+                                  const StepCtl *ctl, int mask, const int *__restrict__ perm, const double *Vbase,
+                                  int vmul, double *xp)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    pdl_wait();   // the stage kernel that makes V
     if (e >= Ntot) return;
     const int i = inst_of[e];
     if (!takes_part(ctl, i, mask)) return;
@@ -998,6 +999,7 @@ __global__ void hm_gather_kernel(int64_t Ntot, const int *__restrict__ inst_of,
                                  const double *__restrict__ out, double *partT, double *partN)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    pdl_trigger();   // the stage kernel's work before its wait runs beside this one
     if (e >= Ntot) return;
     const int c = blockIdx.y;
     const int i = inst_of[e];
