@@ -514,7 +514,7 @@ def leg_tensor_core(args, local, stream, t_end=200.0, n_steps=20):
     """Shared-geometry ensemble: 64 realisations of the 800-fault network
     (per-member a, b, initial V and stepped fault) sharing one kernel matrix,
     so the K.V of all members in a stage is one GEMM streaming K once. The
-    FP64 shared-K batch (FP64 products and sums on the CUDA cores) against
+    FP64 shared-K batch (FP64 products and sums) against
     the BF16 hi+lo tcgen05 batch (FP32 accumulation), in the V formulation
     and the Newton formulation (with and without the learned guess, trained
     on solves recorded from eight members): network-steps/s, time to

@@ -53,9 +53,9 @@ enum { DFN_KERNEL_DIRECT = 0, DFN_KERNEL_HMATRIX = 1 };        /* hyperparameter
  * up to 256 networks), K is stored once as BF16 hi + lo matrices and the
  * K.V of all networks of a stage is one tcgen05 tensor-core GEMM (BF16
  * products, FP32 accumulation). DFN_STORE_FP64_SHARED: the same shared K
- * in FP64 and an FP64 GEMM on the CUDA cores (K streamed once per stage for
- * all networks, products and sums in FP64), the counterpart that isolates
- * the tensor-core arithmetic from the sharing. No counterpart in the
+ * in FP64 and a GEMM on the FP64 matrix instructions (K streamed once per
+ * stage for all networks, products and sums in FP64), the counterpart that
+ * isolates the BF16 arithmetic from the sharing. No counterpart in the
  * reference. */
 enum { DFN_STORE_FP64 = 0, DFN_STORE_FP32 = 1, DFN_STORE_BF16X2 = 2, DFN_STORE_BF16X2_TC = 3,
        DFN_STORE_FP64_SHARED = 4 };
@@ -239,7 +239,8 @@ int32_t dfn_create(const dfn_problem *prob, const dfn_options *opt, dfn_handle *
  * with a 2-stage ring (two CTAs per SM; gemv_impl 2, ms[4], timed when it
  * differs from the deepest ring); all give identical results.
  * CG pressure (DFN_PRESSURE_CG): the stage systems of the batch solved by one
- * CTA each on global memory (ms[2]), by a cluster of CTAs each with the
+ * CTA each on global memory (ms[2]; batches whose systems all have at most
+ * 2048 elements: the same sums with the vectors in registers), by a cluster of CTAs each with the
  * vectors in shared memory (ms[3]; handles with systems of 2048 elements or
  * more) or by one CTA each with the vectors in shared memory (ms[5]; larger
  * systems of the batch on global memory); cg_cluster = 0, 1 or 2 names the
@@ -284,7 +285,8 @@ int32_t dfn_set_wait_limit(dfn_handle *h, int32_t polls);
 /* Form of the CG pressure solves (DFN_PRESSURE_CG handles): -1 the default
  * rule (clusters when a launch's clusters all fit on the GPU at once, else
  * one CTA per system on global memory), 0 one CTA per system on global
- * memory, 1 one thread-block cluster per system with shared-memory vectors
+ * memory (systems of up to 2048 elements: in registers, identical results),
+ * 1 one thread-block cluster per system with shared-memory vectors
  * (systems of 2048 elements or more), 2 one CTA per system with shared-memory
  * vectors (systems too large for them on global memory). The forms agree to
  * the solver tolerance. dfn_autotune sets the fastest. No counterpart in the
