@@ -2603,11 +2603,21 @@ int32_t dfn_get_state_instance(dfn_handle *h, int32_t i, double *Y, double *P, d
     if (!h || i < 0 || i >= h->B) return DFN_ERR_ARG;
     CK(cudaSetDevice(h->dev));
     const Inst &I = h->hinst[i];
+    const size_t nY = sizeof(double) * 3 * (size_t)I.N, nP = sizeof(double) * (size_t)I.N;
     StageScope scope(h);
     TRY(stage_begin(h));
-    if (Y) TRY(get_host(h, Y, h->Y + 3 * I.eoff, sizeof(double) * 3 * I.N));
-    if (P) TRY(get_host(h, P, h->P + I.eoff, sizeof(double) * I.N));
-    TRY(sync_ctl(h));
+    // a state behind an expired wait is not handed out: staged copies are
+    // delivered, and others made, once the flag is known to be clear
+    const bool staged = nY + nP + 128 <= h->stage_size && (!Y || is_pageable(Y)) && (!P || is_pageable(P));
+    if (!staged) TRY(sync_ctl(h));
+    if (Y) TRY(get_host(h, Y, h->Y + 3 * I.eoff, nY));
+    if (P) TRY(get_host(h, P, h->P + I.eoff, nP));
+    if (staged) {
+        TRY(sync_ctl(h, false));
+    } else {
+        CK(cudaStreamSynchronize(h->stream));
+    }
+    stage_end(h);
     if (time) *time = h->h_ctl[i].time;
     if (t_try) *t_try = h->h_ctl[i].t_try;
     if (it_count) *it_count = h->h_ctl[i].it_count;
