@@ -556,13 +556,16 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     }
     __syncthreads();
     if (warp == TMA_CONSUMERS) {
-        // producer: one elected lane issues the bulk copies (it reads nothing
-        // that a kernel writes, so it does not wait for the previous one)
+        // producer: one elected lane issues the bulk copies. K is constant, so
+        // the first ring of them does not wait for the previous kernel; the
+        // bounded waits for a free stage do, since the consumers free none
+        // before it has ended: the limit is on this kernel's own progress
         if (lane == 0) {
             const uint64_t policy = (int64_t)blockIdx.x < keep_tiles ? l2_policy_last() : l2_policy_first();
             int i = 0;
             for (; i < nrows; i++) {
                 int s = i % TMA_STAGES;
+                if (early && i == TMA_STAGES) pdl_wait();
                 if (i >= TMA_STAGES && !mbar_wait(&empty[s], ((i / TMA_STAGES) - 1) & 1, wait_polls)) {
                     bad_s = 1;
                     break;
