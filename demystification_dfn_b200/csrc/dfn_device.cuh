@@ -559,20 +559,26 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
         // producer: one elected lane issues the bulk copies. K is constant, so
         // the first ring of them does not wait for the previous kernel; the
         // bounded waits for a free stage do, since the consumers free none
-        // before it has ended: the limit is on this kernel's own progress
+        // before it has ended: the limit is on this kernel's own progress.
+        // (Two loops: with the wait inside one the K.V back to back took
+        // 17.0 us for 125 MB, with none 15.8, now 15.4.)
         if (lane == 0) {
             const uint64_t policy = (int64_t)blockIdx.x < keep_tiles ? l2_policy_last() : l2_policy_first();
-            int i = 0;
-            for (; i < nrows; i++) {
-                int s = i % TMA_STAGES;
-                if (early && i == TMA_STAGES) pdl_wait();
-                if (i >= TMA_STAGES && !mbar_wait(&empty[s], ((i / TMA_STAGES) - 1) & 1, wait_polls)) {
-                    bad_s = 1;
-                    break;
-                }
+            auto copy = [&](int i, int s) {
                 mbar_expect_tx(&full[s], GEMV_CHUNK_BYTES);
                 tma_bulk_g2s_hint(stage + s * (GEMV_CHUNK_BYTES / 16), K + (r0 + i) * row_bytes + c * GEMV_CHUNK_BYTES,
                                   GEMV_CHUNK_BYTES, &full[s], policy);
+            };
+            int i = 0;
+            for (; i < nrows && i < TMA_STAGES; i++) copy(i, i);
+            if (early && i < nrows) pdl_wait();
+            for (; i < nrows; i++) {
+                const int s = i % TMA_STAGES;
+                if (!mbar_wait(&empty[s], ((i / TMA_STAGES) - 1) & 1, wait_polls)) {
+                    bad_s = 1;
+                    break;
+                }
+                copy(i, s);
             }
             issued_s = i;
         }
