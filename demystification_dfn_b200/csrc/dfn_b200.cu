@@ -12,6 +12,7 @@
 // and reads the controllers only between groups of rounds.
 #include "../../include/dfn_b200.h"
 #include "dfn_device.cuh"
+#include "kv_l2.cuh"
 #include "hmat_device.cuh"
 #include "newton.cuh"
 #include "tc_gemm.cuh"
@@ -101,7 +102,7 @@ struct dfn_handle {
     int *inst_of = nullptr;
     int4 *tiles = nullptr;
     int64_t ntiles = 0, ntiles0 = 0;      // all tiles / tiles of network 0
-    int64_t keep_tiles = 0;               // the first ones stay in L2 from one K.V to the next
+    int64_t keep_tiles = -1;              // the first ones stay in L2 from one K.V to the next (-1: no policy)
     int64_t *seg_start = nullptr;
     int *seg_inst = nullptr;
     int64_t nseg = 0, nseg0 = 0;
@@ -1450,19 +1451,6 @@ static int gemv_rows(const std::vector<Inst> &inst, int64_t slots)
     return rows;
 }
 
-// Tiles of the dense K.V that stay in L2 from one K.V to the next: kL2Keep
-// bytes of a matrix that does not fit (what the policies give beyond is more
-// than half of L2's 126 MB away from the vectors), none of a smaller one,
-// which stays by itself. 16 steps, no policy / all copies evict-first / 48 MB
-// kept: 128 MB of K 2.95 / 2.24 / 2.11 ms, 152 MB 4.12 / 3.54 / 3.42, 256 MB
-// 5.05 / 4.59 / 4.36, 716 MB 13.9 / 13.0 / 12.7, 2.3 GB 38.2 / 36.7 / 36.7;
-// 32 and 64 MB are within 2 % of 48, from 96 MB on the gain is gone.
-static const int64_t kL2Keep = (int64_t)48 << 20, kL2Fits = (int64_t)64 << 20;
-static int64_t l2_keep_tiles(int64_t ntiles, int64_t bytes)
-{
-    return bytes <= kL2Fits ? 0 : (int64_t)((double)ntiles * (double)kL2Keep / (double)bytes);
-}
-
 static int single_only(const dfn_handle *h)
 {
     if (h->B != 1) {
@@ -2064,7 +2052,7 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
         if (i == 0) h->ntiles0 = (int64_t)tiles.size();
     }
     h->ntiles = (int64_t)tiles.size();
-    h->keep_tiles = l2_keep_tiles(h->ntiles, h->kv_bytes);
+    h->keep_tiles = l2_keep_tiles(h->ntiles, [&](int64_t q) { return (int64_t)tiles[q].w * GEMV_CHUNK_BYTES; });
     DALLOC(h->tiles, tiles.size());
     if (!tiles.empty()) HCOPY(h->tiles, tiles.data(), tiles.size());
     PressGlobal &pg = h->pg;

@@ -493,6 +493,12 @@ __device__ __forceinline__ uint64_t l2_policy_last()
     asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
+__device__ __forceinline__ uint64_t l2_policy_normal()
+{
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
 __device__ __forceinline__ uint64_t l2_policy_first()
 {
     uint64_t p;
@@ -505,10 +511,10 @@ __device__ __forceinline__ uint64_t l2_policy_first()
 // shared memory completed on mbarriers; eight consumer warps read the stages
 // with 128-bit shared loads. Rows of the tile go to consumer warps
 // round-robin, one stage per row (stage s is always read by warp s % 8).
-// The matrices are read over and over, K.V after K.V, and least-recently-used
-// replacement keeps nothing of what is larger than L2: the copies of the
-// first keep_tiles tiles stay in L2 (evict_last), the others pass through it
-// (evict_first), also past the vectors that the stage kernel reads.
+// The matrices are read over and over, K.V after K.V: with keep_tiles >= 0
+// the copies of the first keep_tiles tiles stay in L2 (evict_last) and the
+// others pass through it (evict_first), also past the vectors that the stage
+// kernel reads; keep_tiles < 0: no policy (kv_l2.cuh).
 template <int MODE, int STORE>
 __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     gemv_tma_kernel(const int4 *__restrict__ tiles, const Inst *__restrict__ inst, const StepCtl *ctl,
@@ -563,7 +569,8 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
         // (Two loops: with the wait inside one the K.V back to back took
         // 17.0 us for 125 MB, with none 15.8, now 15.4.)
         if (lane == 0) {
-            const uint64_t policy = (int64_t)blockIdx.x < keep_tiles ? l2_policy_last() : l2_policy_first();
+            const uint64_t policy = keep_tiles < 0 ? l2_policy_normal()
+                                    : (int64_t)blockIdx.x < keep_tiles ? l2_policy_last() : l2_policy_first();
             auto copy = [&](int i, int s) {
                 mbar_expect_tx(&full[s], GEMV_CHUNK_BYTES);
                 tma_bulk_g2s_hint(stage + s * (GEMV_CHUNK_BYTES / 16), K + (r0 + i) * row_bytes + c * GEMV_CHUNK_BYTES,
