@@ -103,6 +103,7 @@ struct dfn_handle {
     int4 *tiles = nullptr;
     int64_t ntiles = 0, ntiles0 = 0;      // all tiles / tiles of network 0
     int64_t keep_tiles = -1;              // the first ones stay in L2 from one K.V to the next (-1: no policy)
+    bool l2_kept = false;                 // a K.V has been launched that keeps them
     int64_t *seg_start = nullptr;
     int *seg_inst = nullptr;
     int64_t nseg = 0, nseg0 = 0;
@@ -487,6 +488,7 @@ static int launch_gemv(dfn_handle *h, int mask, const double *Vbase, int vmul, b
         TRY(launch_s64(h, mask, Vbase, vmul));
     } else if (h->gemv_impl == 0) {
         gemv_tma_fn fn = pick_gemv_tma(h->mode, h->store);
+        h->l2_kept = h->keep_tiles > 0;
         CK(launch_pdl(fn, (unsigned)ntiles, (TMA_CONSUMERS + 1) * 32, kTmaSmem, h->stream, h->tiles, h->inst, h->ctl,
                       mask, K, Vbase, vmul, h->partT, h->partN, h->wait_polls, h->err_flag, h->keep_tiles));
     } else {
@@ -1502,6 +1504,11 @@ int32_t dfn_destroy(dfn_handle *h)
     if (!h) return DFN_OK;
     cudaSetDevice(h->dev);
     if (h->stream) cudaStreamSynchronize(h->stream);
+    if (h->l2_kept) {
+        l2_release_kernel<<<(unsigned)h->keep_tiles, 256, 0, h->stream>>>(
+            h->tiles, h->inst, static_cast<const unsigned char *>(h->K), bytes_per_col(h->mode, h->store));
+        cudaStreamSynchronize(h->stream);
+    }
     void *ptrs[] = {h->kstar, h->kmin, h->Snk, h->s64_vt, h->slip, h->slip_out, h->slip_acc, h->tau0, h->wlast, h->vnow, h->mlp, h->rec_x, h->rec_t, h->rec_n,
                     h->hblk, h->ht1, h->ht2, h->hvals, h->hperm, h->hsegof, h->hsegptr, h->hsegbase, h->hz, h->hout, h->hxp, h->ht3, h->htg, h->hdg, h->hdl, h->hl4, h->hl5, h->hlw, h->xptr, h->xcon, h->xrows, h->xrows_ptr, h->tri_tiles, h->tcoef,
                     h->inst, h->inst_of, h->tiles, h->seg_start, h->seg_inst, h->long_seg, h->short_seg, h->tc_A, h->tc_B, h->node, h->elem, h->ds, h->tan,

@@ -632,6 +632,24 @@ __global__ void __launch_bounds__((TMA_CONSUMERS + 1) * 32)
     }
 }
 
+// Gives the kept share of L2 back when a handle ends: the lines of the kept
+// tiles (a CTA each) lose their priority. Left as they are they go on pushing
+// others' lines out after the matrix is freed: the next 75 reads of a 90 MiB
+// array took 22.4 -> 29.8 us, 23.2 with this.
+__global__ void l2_release_kernel(const int4 *__restrict__ tiles, const Inst *__restrict__ inst,
+                                  const unsigned char *Kbase, int bytes_per_col)
+{
+    constexpr int LINE = 128, LINES = GEMV_CHUNK_BYTES / LINE;
+    const int4 t = tiles[blockIdx.x];
+    const Inst &I = inst[t.x];
+    const int64_t row_bytes = I.Np * bytes_per_col;
+    const unsigned char *K = Kbase + I.kvec * 16 + t.z * row_bytes + (int64_t)t.y * GEMV_CHUNK_BYTES;
+    for (int q = threadIdx.x; q < t.w * LINES; q += blockDim.x)
+        asm volatile("applypriority.global.L2::evict_normal [%0], 128;" ::"l"(K + q / LINES * row_bytes +
+                                                                              q % LINES * LINE)
+                     : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Pore pressure (src/fluid_diffusion.f90). The parameters of the implicit
 // step are shared by both solvers.

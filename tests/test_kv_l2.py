@@ -5,6 +5,7 @@ import subprocess
 import pytest
 
 from demystification_dfn_b200 import networks
+from demystification_dfn_b200.ensemble import Ensemble
 from demystification_dfn_b200.simulation import Simulation
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -80,3 +81,40 @@ def test_small_matrix_beside_a_kept_share():
                 large.time_kernel(20)
                 beside = min(beside, small.time_kernel(50))
     assert beside <= 1.2 * alone
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,storage,n,count", [("modeII", "fp64", 4000, 1), ("modeIII", "bf16x2", 1500, 30)])
+def test_kept_share_ends_with_the_handle(mode, storage, n, count):
+    """Reads of a 90 MiB array, which L2 holds, before a handle with a kept
+    share and after its end: alike, so at most 1.1 times (1.3 when the kept
+    lines stay behind, which it takes about 75 reads to push out). The median
+    of 25 reads on both sides, the best of three handles."""
+    import torch
+
+    x = torch.zeros(90 << 18, dtype=torch.float32, device="cuda")
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+
+    def reads():
+        t = []
+        for _ in range(25):
+            a.record()
+            x.sum()
+            b.record()
+            b.synchronize()
+            t.append(a.elapsed_time(b))
+        return sorted(t[2:])[11]
+
+    other = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    p = networks.single_fault(n_el=n, length=10.0 * n, mode=mode)
+    ratios = []
+    for _ in range(3):
+        for k in range(4):
+            other.fill_(k)      # whatever was kept before is gone
+        reads()
+        before = reads()
+        e = Ensemble([p] * count, storage=storage, pressure="tridiag")
+        e.time_kernel(20)
+        e.close()
+        ratios.append(reads() / before)
+    assert min(ratios) <= 1.1, ratios
