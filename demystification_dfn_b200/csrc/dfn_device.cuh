@@ -92,10 +92,13 @@ __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a,
 // Programmatic dependent launch. A kernel launched with the attribute may
 // start while the kernel before it on the stream still runs; pdl_wait()
 // returns once that kernel has completed and its writes are visible, and
-// pdl_trigger() lets the next kernel start. Every kernel calls wait, then
-// trigger, in every block before it returns: when a kernel's wait returns,
-// all kernels before the previous one have completed too, so what comes
-// before the wait may read anything but the previous kernel's results.
+// pdl_trigger() lets the next kernel start. A kernel that triggers waits
+// first, in every block, and a kernel launched with the attribute waits in
+// every block before it returns, whether it triggers or not (its end does
+// then): so when a kernel's wait returns, all kernels before the previous one
+// have completed too, and what comes before the wait may read anything but
+// the previous kernel's results. Kernels without either call are launched
+// without the attribute.
 // Without the attribute the wait returns at once. What an earlier kernel of
 // the chain writes is no __restrict__ const parameter here: such loads count
 // as invariant and may be moved before the wait.

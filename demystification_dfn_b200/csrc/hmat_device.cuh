@@ -999,6 +999,7 @@ __global__ void hm_gather_kernel(int64_t Ntot, const int *__restrict__ inst_of,
                                  const double *__restrict__ out, double *partT, double *partN)
 {
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    pdl_wait();      // returns at once in a launch without the attribute, as after the join of the leaf streams
     pdl_trigger();   // the stage kernel's work before its wait runs beside this one
     if (e >= Ntot) return;
     const int c = blockIdx.y;
