@@ -790,7 +790,8 @@ static int run_round(dfn_handle *h)
 // controllers and the error flag) serves them all. Pinned buffers of the
 // caller are copied directly, and so is what the staging memory cannot hold.
 // Every entry point that stages starts with a StageScope and stage_begin and
-// ends with sync_ctl. K.V call at N = 6 691: 200 -> 178 us, right-hand side at
+// ends with sync_ctl; those that leave the caller's buffers alone on failure
+// look at the flag or status before stage_end. K.V call at N = 6 691: 200 -> 178 us, right-hand side at
 // N = 1 404: 124 -> 82 us, 4 steps with host buffers at N = 4 361: 4.15 -> 3.79 ms.
 static const size_t kStageMax = (size_t)4 << 20;
 
@@ -1437,7 +1438,8 @@ static int build_hmatrix(dfn_handle *h, const dfn_problem *probs, const dfn_opti
 // FP64 13.4 -> 4.2 us, 1404 mode III FP32 14.4 -> 8.2, 2000 mode II FP64 14.4
 // -> 10.3, 4000 mode III FP64 32 -> 26, FP32 16.5 -> 14.4, 4361 mode III FP32
 // 26.7 -> 20.2; every other multiple of 8 up to 128 is at best 6 % faster
-// (N = 100 to 6691). From eight waves on all heights are within 3 %.
+// (N = 100 to 6691). From eight waves on all heights are within 3 %. (Times
+// before the copies of K started ahead of the launch and kept a share in L2.)
 static int gemv_rows(const std::vector<Inst> &inst, int64_t slots)
 {
     auto ntiles = [&](int rows) {

@@ -2238,7 +2238,9 @@ __device__ __forceinline__ void newton_post(const FricParams &f, int64_t e, doub
 // log-state, pressure and normal traction give by themselves, then what needs
 // the stress rates (src/friction/RateStateAgingModeII.f90:46-76; mode III:
 // dsig = loading only). Operations are written out (no contraction left to
-// the compiler), so that every instantiation of the stage kernel rounds alike.
+// the compiler), so that every instantiation of the stage kernel rounds alike
+// (those of the Newton formulation are not: there the variants for small and
+// large launches agree bit for bit as they are compiled).
 struct RsfPre {
     double as;       // a asinh(B C)
     double w;        // B D (sig + P) b heal

@@ -7,10 +7,10 @@
 // isolate what the BF16 hi+lo arithmetic itself gains. (The reference has one
 // network per process and no batch.)
 //
-// The products run on the FP64 matrix instructions (mma.sync m16n8k16.f64:
+// The products run on the FP64 matrix instructions (mma.sync m16n8k4.f64:
 // IEEE FP64 products and sums): the contraction is bound by the FP64 unit for
 // R >= 16 (16 flop per byte of K at R = 64), and against scalar FMAs one
-// instruction replaces 64 per lane and a fragment load serves 16 rows x 8
+// instruction replaces 16 per lane and a fragment load serves 16 rows x 8
 // members.
 //
 // K is stored row-major, N rows of Np columns (Np = N padded to S64_COLS with
@@ -20,8 +20,8 @@
 // member tile; NT the smallest that covers R in the fewest tiles, so that
 // padding costs at most 7 members per tile) and streams the columns in chunks
 // of S64_COLS through a ring of shared-memory stages (cp.async, 16 bytes per
-// copy). Lane (g, t) of a warp holds rows g, g + 8 and columns t, t + 4,
-// t + 8, t + 12 of the chunk, which is the fragment order of the instruction;
+// copy). A chunk is four instructions per member tile and component: in the
+// j-th, lane (g, t) of a warp holds rows g, g + 8 of column t + 4 j;
 // the stage rows are padded so that a quarter-warp's 16-byte reads of K and a
 // half-warp's 8-byte reads of V cover all banks once.
 //

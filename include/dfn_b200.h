@@ -278,7 +278,8 @@ int32_t dfn_set_graphs(dfn_handle *h, int32_t enable);
  * with the full limit for its own copies in flight, raises an error flag
  * and returns; the next call that reads the step controllers returns
  * DFN_ERR_TIMEOUT once (the partial sums of that K.V are incomplete, so the
- * state must be restored, e.g. with dfn_set_state). polls < 0 restores the
+ * state must be restored, e.g. with dfn_set_state). The limit is on the K.V's
+ * own progress, not on the kernel before it. polls < 0 restores the
  * default (2^22 polls, far beyond any copy's latency); 0 gives up at the
  * first wait, which tests the error path. No counterpart in the reference. */
 int32_t dfn_set_wait_limit(dfn_handle *h, int32_t polls);
