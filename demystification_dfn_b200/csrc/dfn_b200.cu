@@ -793,7 +793,13 @@ static int run_round(dfn_handle *h)
 // ends with sync_ctl; those that leave the caller's buffers alone on failure
 // look at the flag or status before stage_end. K.V call at N = 6 691: 200 -> 178 us, right-hand side at
 // N = 1 404: 124 -> 82 us, 4 steps with host buffers at N = 4 361: 4.15 -> 3.79 ms.
-static const size_t kStageMax = (size_t)4 << 20;
+// Beyond a megabyte pinned memory takes 1 to 2.5 ms to allocate and 2 ms to
+// give back (N = 16 013: 1.2 MB, creation 9.6 -> 12 ms, closing 4.2 -> 6.1),
+// below nothing that shows, and more of it gives nothing: state / snapshot /
+// step at N = 16 013 54 / 99 / 1627 us with 768 KB, 54 / 98 / 1626 with 1.2 MB,
+// 73 / 135 / 1647 with 256 KB. Larger uploads than 256 KB are copied by the
+// driver in pieces and are faster so (N = 60 000: 262 us against 270 to 297).
+static const size_t kStageMax = (size_t)768 << 10, kStageUpload = (size_t)256 << 10;
 
 static bool is_pageable(const void *p)
 {
@@ -833,7 +839,7 @@ static char *stage_take(dfn_handle *h, size_t bytes)
 
 static int put_host(dfn_handle *h, void *dev, const void *host, size_t bytes)
 {
-    char *p = is_pageable(host) ? stage_take(h, bytes) : nullptr;
+    char *p = bytes <= kStageUpload && is_pageable(host) ? stage_take(h, bytes) : nullptr;
     if (p) memcpy(p, host, bytes);
     CK(cudaMemcpyAsync(dev, p ? p : host, bytes, cudaMemcpyHostToDevice, h->stream));
     return DFN_OK;

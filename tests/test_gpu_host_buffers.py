@@ -114,10 +114,10 @@ def test_buffers_of_either_kind_get_the_same(n_el):
             assert np.array_equal(ref[k], got[k]), k
 
 
-def test_buffers_larger_than_the_staging_memory():
-    """140 000 elements: the state (4.5 MB) does not fit the staging memory, its
-    pressure does, single vectors do, a step's do in part."""
-    n = 140_000
+@pytest.mark.parametrize("n", [20_000, 30_000, 140_000])
+def test_buffers_larger_than_the_staging_memory(n):
+    """20 000 elements: the state fits the staging memory, a step's vectors do in
+    part; 30 000: the state does not, single vectors do; 140 000: none does."""
     p = networks.single_fault(n_el=n, length=10.0 * n, mode="modeIII", kernel="hmatrix", tol=1e-6)
     kw = dict(pressure="tridiag", storage="fp32", hmat_leaf=64, hmat_eta=2.0, hmat_eps=1e-4)
     ref, got = (_all_calls(p, pinned, **kw) for pinned in (True, False))
