@@ -17,13 +17,13 @@
 // zero columns), {K_T, K_N} per column in mode II; the V of all members is
 // packed per stage into vt[m][l] (members padded to 8, columns to Np, zeros).
 // A CTA of four warps takes S64_ROWS rows (16 per warp) x 8 NT members (a
-// member tile; NT the smallest that covers R in the fewest tiles, so that
-// padding costs at most 7 members per tile) and streams the columns in chunks
-// of S64_COLS through a ring of shared-memory stages (cp.async, 16 bytes per
-// copy). A chunk is four instructions per member tile and component: in the
-// j-th, lane (g, t) of a warp holds rows g, g + 8 of column t + 4 j;
-// the stage rows are padded so that a quarter-warp's 16-byte reads of K and a
-// half-warp's 8-byte reads of V cover all banks once.
+// member tile; NT the smallest that covers R in as few tiles as fill the GPU,
+// so that padding costs at most 7 members per tile) and streams the columns in
+// chunks of S64_COLS through a ring of shared-memory stages (cp.async, 16
+// bytes per copy). A chunk is four instructions per group of eight members and
+// component: in the j-th, lane (g, t) of a warp holds rows g, g + 8 of column
+// t + 4 j. The stage rows are padded so that a quarter-warp's 16-byte reads of
+// K and a half-warp's 8-byte reads of V cover all banks once.
 //
 // Split of the work: the (row tile, member tile, column chunk) steps form one
 // sequence that the CTAs of a single wave share evenly (CTA b takes steps
@@ -51,6 +51,13 @@ constexpr int S64_NT = 8;                        // at most 8 tiles of 8 members
 // are spread thin: N = 305, R = 43 takes 31 / 16.5 / 14.5 / 14.4 us with 8 / 4
 // / 2 / 1 (one only adds partial sums); from N = 2000 on no difference.
 constexpr int S64_MIN_STEPS = 2;
+// Steps per SM below which the member tiles are narrowed: a small matrix with
+// wide tiles is a few CTAs of long steps. K.V in us, scalar FMAs before / the
+// fewest tiles / this rule, mode II: N = 100, R = 64 12.5 / 18.6 / 6.3; 200,
+// 128 13.3 / 21.2 / 8.3; 305, 256 20.6 / 15.8 / 13.7; 450, 192 24.7 / 28.4 /
+// 18.8; 1000, 64 34.9 / 26.3 / 20.5. With 1, 2 or 4 some of these gain less or
+// nothing (450, 192: 28.4 / 29.6 / 28.6).
+constexpr int S64_FILL = 8;
 constexpr int S64_VROW = S64_COLS + 4;           // doubles of a staged V row (160 bytes)
 
 // doubles of a staged K row: 320 bytes (mode II) or 160
@@ -93,11 +100,14 @@ inline S64Plan s64_plan(int64_t N, int R, int sms)
 {
     S64Plan p;
     const int n8 = (R + 7) / 8;
-    p.mtiles = (n8 + S64_NT - 1) / S64_NT;
-    p.nt = (n8 + p.mtiles - 1) / p.mtiles;
     p.nkc = (int)((N + S64_COLS - 1) / S64_COLS);
     p.rtiles = (int)((N + S64_ROWS - 1) / S64_ROWS);
-    p.steps = (int64_t)p.rtiles * p.mtiles * p.nkc;
+    for (int tiles = (n8 + S64_NT - 1) / S64_NT;; tiles++) {
+        p.nt = (n8 + tiles - 1) / tiles;
+        p.mtiles = (n8 + p.nt - 1) / p.nt;
+        p.steps = (int64_t)p.rtiles * p.mtiles * p.nkc;
+        if (p.nt == 1 || p.steps >= (int64_t)S64_FILL * sms) break;
+    }
     p.ctas = p.steps / S64_MIN_STEPS < 1 ? 1 : p.steps / S64_MIN_STEPS;
     if (p.ctas > 2 * (int64_t)sms) p.ctas = 2 * (int64_t)sms;
     for (int64_t t = 0; t < (int64_t)p.rtiles * p.mtiles; t++) {
