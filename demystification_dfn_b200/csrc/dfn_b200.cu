@@ -2041,8 +2041,11 @@ int32_t dfn_create_batch(const dfn_problem *probs, int32_t count, const dfn_opti
     int tile_rows = GEMV_ROWS;
     if (!h->hmat && !h->tc && !h->s64) {
         int per_sm = 0;
-        CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_gemv_tma(h->mode, h->store),
-                                                          (TMA_CONSUMERS + 1) * 32, kTmaSmem));
+        if (h->gemv_impl == 0)
+            CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_gemv_tma(h->mode, h->store),
+                                                              (TMA_CONSUMERS + 1) * 32, kTmaSmem));
+        else
+            CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pick_gemv(h->mode, h->store), GEMV_WARPS * 32, 0));
         tile_rows = gemv_rows(h->hinst, (int64_t)std::max(per_sm, 1) * h->sms);
     }
     for (int i = 0; i < count && !h->hmat && !h->tc && !h->s64; i++) {

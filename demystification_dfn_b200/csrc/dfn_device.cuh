@@ -372,6 +372,11 @@ __device__ __forceinline__ bool press_takes_part(const StepCtl *ctl, int i, int 
 // in flight). The per-(chunk,row) warp sum goes to part[c*N + row]; the
 // consumer adds the chunks in a fixed order, so the result is deterministic.
 // V of instance i is Vbase[vmul*eoff_i + l].
+// AHEAD: the first two rows are loaded before V and the next two before the
+// sums of these. 16-byte columns, N = 2117 / 4000 / 9000: 17 / 52 / 201 ->
+// 11 / 41 / 188 us; 4-byte columns, BF16, 3000 / 6000 / 9000: 12.4 / 61 / 131 ->
+// 9.5 / 34 / 70 us. With 8-byte columns the registers cost more than that
+// gives (N = 4000 / 9000 23 / 107 -> 31 / 129 us).
 template <int MODE, int STORE>
 __global__ void __launch_bounds__(GEMV_WARPS * 32)
     gemv_kernel(const int4 *__restrict__ tiles, const Inst *__restrict__ inst, const StepCtl *__restrict__ ctl,
@@ -381,6 +386,7 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32)
     constexpr int BPC = KFmt<MODE, STORE>::BPC;
     constexpr int CPV = 16 / BPC;                 // columns per 16-byte vector
     constexpr int CW = GEMV_CHUNK_BYTES / BPC;    // columns per chunk
+    constexpr bool AHEAD = CPV != 2;
     const int4 t = tiles[blockIdx.x];
     if (!takes_part(ctl, t.x, mask)) return;
     const Inst I = inst[t.x];
@@ -393,6 +399,17 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32)
     const int64_t r0 = t.z, rend = r0 + t.w;
     const int64_t row_vecs = I.Np * BPC / 16;
 
+    const int64_t vec0 = c * (CW * BPC / 16) + lane;
+    uint4 qa[GEMV_LPL], qb[GEMV_LPL];
+    auto load = [&](int64_t r) {   // rows r and r + GEMV_WARPS (r again where that is not in the tile)
+        const uint4 *pa = K + r * row_vecs + vec0, *pb = pa + (r + GEMV_WARPS < rend ? GEMV_WARPS * row_vecs : 0);
+#pragma unroll
+        for (int i = 0; i < GEMV_LPL; i++) qa[i] = __ldcs(pa + i * 32);
+#pragma unroll
+        for (int i = 0; i < GEMV_LPL; i++) qb[i] = __ldcs(pb + i * 32);
+    };
+    int64_t r = r0 + warp;
+    if (AHEAD && r < rend) load(r);
     double v[GEMV_LPL * CPV];
 #pragma unroll
     for (int i = 0; i < GEMV_LPL; i++)
@@ -402,22 +419,23 @@ __global__ void __launch_bounds__(GEMV_WARPS * 32)
             v[i * CPV + j] = (col < N) ? Vin[col] : 0.0;
         }
 
-    const int64_t vec0 = c * (CW * BPC / 16) + lane;
-    for (int64_t r = r0 + warp; r < rend; r += 2 * GEMV_WARPS) {
+    for (; r < rend; r += 2 * GEMV_WARPS) {
         const int64_t rb = r + GEMV_WARPS;
         const bool two = rb < rend;
-        const uint4 *pa = K + r * row_vecs + vec0;
-        const uint4 *pb = K + (two ? rb : r) * row_vecs + vec0;
-        uint4 qa[GEMV_LPL], qb[GEMV_LPL];
+        if constexpr (!AHEAD) {
+            const uint4 *pa = K + r * row_vecs + vec0;
+            const uint4 *pb = K + (two ? rb : r) * row_vecs + vec0;
 #pragma unroll
-        for (int i = 0; i < GEMV_LPL; i++) qa[i] = __ldcs(pa + i * 32);
+            for (int i = 0; i < GEMV_LPL; i++) qa[i] = __ldcs(pa + i * 32);
 #pragma unroll
-        for (int i = 0; i < GEMV_LPL; i++) qb[i] = two ? __ldcs(pb + i * 32) : make_uint4(0, 0, 0, 0);
+            for (int i = 0; i < GEMV_LPL; i++) qb[i] = two ? __ldcs(pb + i * 32) : make_uint4(0, 0, 0, 0);
+        }
         double aT = 0.0, aN = 0.0, bT = 0.0, bN = 0.0;
 #pragma unroll
         for (int i = 0; i < GEMV_LPL; i++) fma_vec<MODE, STORE>(qa[i], v + i * CPV, aT, aN);
 #pragma unroll
         for (int i = 0; i < GEMV_LPL; i++) fma_vec<MODE, STORE>(qb[i], v + i * CPV, bT, bN);
+        if (AHEAD && r + 2 * GEMV_WARPS < rend) load(r + 2 * GEMV_WARPS);
         aT = warp_sum(aT); bT = warp_sum(bT);
         if (MODE == 2) { aN = warp_sum(aN); bN = warp_sum(bN); }
         if (lane == 0) {
