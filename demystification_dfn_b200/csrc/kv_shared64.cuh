@@ -51,13 +51,17 @@ constexpr int S64_NT = 8;                        // at most 8 tiles of 8 members
 // are spread thin: N = 305, R = 43 takes 31 / 16.5 / 14.5 / 14.4 us with 8 / 4
 // / 2 / 1 (one only adds partial sums); from N = 2000 on no difference.
 constexpr int S64_MIN_STEPS = 2;
-// Steps per SM below which the member tiles are narrowed: a small matrix with
-// wide tiles is a few CTAs of long steps. K.V in us, scalar FMAs before / the
-// fewest tiles / this rule, mode II: N = 100, R = 64 12.5 / 18.6 / 6.3; 200,
-// 128 13.3 / 21.2 / 8.3; 305, 256 20.6 / 15.8 / 13.7; 450, 192 24.7 / 28.4 /
-// 18.8; 1000, 64 34.9 / 26.3 / 20.5. With 1, 2 or 4 some of these gain less or
-// nothing (450, 192: 28.4 / 29.6 / 28.6).
-constexpr int S64_FILL = 8;
+// Steps per SM below which the member tiles are narrowed, and the groups of
+// eight members up to which one tile takes them all: a small matrix with wide
+// tiles is a few CTAs of long, unevenly shared steps. K.V in us, scalar FMAs
+// before / the fewest tiles / this rule, mode II: N = 100, R = 64 12.5 / 18.6 /
+// 6.6; 200, 128 13.3 / 21.2 / 8.4; 450, 192 24.7 / 27.0 / 18.8; 1150, 64 34.9 /
+// 40.7 / 22; 1386, 64 43.2 / 45.8 / 30.9. No size from 39 to 4000 with 2 to 256
+// members is slower than with the scalar FMAs; with 8 steps 1150, 64 is, with
+// 12 1386, 64, and with 16 or 24, or fewer groups narrowed too, others lose
+// what these gain (1500, 17 15.5 -> 16.7; 850, 130 29.6 -> 33.5).
+constexpr int S64_FILL = 14;
+constexpr int S64_WHOLE = 4;
 constexpr int S64_VROW = S64_COLS + 4;           // doubles of a staged V row (160 bytes)
 
 // doubles of a staged K row: 320 bytes (mode II) or 160
@@ -106,7 +110,7 @@ inline S64Plan s64_plan(int64_t N, int R, int sms)
         p.nt = (n8 + tiles - 1) / tiles;
         p.mtiles = (n8 + p.nt - 1) / p.nt;
         p.steps = (int64_t)p.rtiles * p.mtiles * p.nkc;
-        if (p.nt == 1 || p.steps >= (int64_t)S64_FILL * sms) break;
+        if (p.nt == 1 || n8 <= S64_WHOLE || p.steps >= (int64_t)S64_FILL * sms) break;
     }
     p.ctas = p.steps / S64_MIN_STEPS < 1 ? 1 : p.steps / S64_MIN_STEPS;
     if (p.ctas > 2 * (int64_t)sms) p.ctas = 2 * (int64_t)sms;
