@@ -845,9 +845,10 @@ static int put_host(dfn_handle *h, void *dev, const void *host, size_t bytes)
     return DFN_OK;
 }
 
-static int get_host(dfn_handle *h, void *host, const void *dev, size_t bytes)
+// pageable: the caller has asked already
+static int get_host(dfn_handle *h, void *host, const void *dev, size_t bytes, bool pageable = false)
 {
-    char *p = is_pageable(host) ? stage_take(h, bytes) : nullptr;
+    char *p = pageable || is_pageable(host) ? stage_take(h, bytes) : nullptr;
     CK(cudaMemcpyAsync(p ? p : host, dev, bytes, cudaMemcpyDeviceToHost, h->stream));
     if (p) h->owed.push_back({host, p, bytes});
     return DFN_OK;
@@ -2501,8 +2502,8 @@ int32_t dfn_compute_P(dfn_handle *h, double dt, double *P_temp, double *P_dot, i
     // where they fit and delivered once the status is known
     const bool staged = 2 * (sizeof(double) * (size_t)N + 64) <= h->stage_size && is_pageable(P_temp) && is_pageable(P_dot);
     if (staged) {
-        TRY(get_host(h, P_temp, h->Ptemp, sizeof(double) * N));
-        TRY(get_host(h, P_dot, h->Pdot_s, sizeof(double) * N));
+        TRY(get_host(h, P_temp, h->Ptemp, sizeof(double) * N, true));
+        TRY(get_host(h, P_dot, h->Pdot_s, sizeof(double) * N, true));
     }
     TRY(sync_ctl(h, false));
     int st = h->h_ctl[0].status;
@@ -2615,8 +2616,8 @@ int32_t dfn_get_state_instance(dfn_handle *h, int32_t i, double *Y, double *P, d
     // delivered, and others made, once the flag is known to be clear
     const bool staged = nY + nP + 128 <= h->stage_size && (!Y || is_pageable(Y)) && (!P || is_pageable(P));
     if (!staged) TRY(sync_ctl(h));
-    if (Y) TRY(get_host(h, Y, h->Y + 3 * I.eoff, nY));
-    if (P) TRY(get_host(h, P, h->P + I.eoff, nP));
+    if (Y) TRY(get_host(h, Y, h->Y + 3 * I.eoff, nY, staged));
+    if (P) TRY(get_host(h, P, h->P + I.eoff, nP, staged));
     if (staged) {
         TRY(sync_ctl(h, false));
     } else {
